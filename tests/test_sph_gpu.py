@@ -83,6 +83,73 @@ def test_particles_outside_the_grid(cuda, pkg, oracle_mod):
     sim.close()
 
 
+@pytest.mark.parametrize("n,spacing,warp_max", [
+    (12000, 0.035, -1), (12001, 0.035, -1),      # 16 / 8 lanes per particle
+    (22000, 0.035, -1), (22001, 0.035, -1),      # 8 lanes / a thread for the forces
+    (130000, 0.035, -1), (130001, 0.035, -1),    # 8 lanes / a thread for the densities
+    (5000, 0.02, -1), (20000, 0.02, -1),         # more neighbours (180) than a list holds
+    (20000, 0.02, 0), (130001, 0.02, -1),
+])
+def test_density_and_force_variants(cuda, pkg, oracle_mod, n, spacing, warp_max):
+    """Either side of each change of kernel, and lists that overflow in each:
+    a moving block at rest spacing or compressed, some particles at one place
+    (distance 0) and some at rest relative to each other, two substeps."""
+    rng = np.random.default_rng(n)
+    a = int(np.ceil(n ** (1.0 / 3.0)))
+    i = np.arange(n)
+    rec = np.zeros((n, 16), np.float32)
+    rec[:, 0:3] = (np.stack([i % a, (i // a) % a, i // (a * a)], axis=1) - 0.5 * a) * spacing
+    rec[:, 0:3] += 0.2 * spacing * rng.random((n, 3))
+    rec[:, 4:7] = rng.normal(0.0, 0.3, (n, 3))
+    rec[1:20, 0:3] = rec[0, 0:3]
+    rec[100:200, 4:7] = 0.0
+    half = [2.0, 2.0, 2.0]
+    sim = pkg.SPHSimulator(None, None, 0.08, maxParticles=n)
+    sim.warpPerParticle = warp_max
+    sim.upload(rec, half)
+    sim.execute()
+    want, pv = oracle_mod.sph_execute(rec, half, 2)
+    assert_bits_equal(sim.downloadParticles(), want, "records")
+    assert_bits_equal(sim.downloadPosvel(), pv, "posvel")
+    sim.close()
+
+
+@pytest.mark.parametrize("n", [3000, 25000])
+def test_capacity_without_neighbour_lists(cuda, pkg, oracle_mod, n):
+    """A capacity too large for neighbour lists: the forces walk the rows."""
+    recs = pkg.sph_scene_dambreak([1.0, 2.0, 1.0], n, 3)
+    sim = pkg.SPHSimulator(None, None, 0.08, maxParticles=(1 << 23) + 1)
+    sim.upload(recs, [1.0, 2.0, 1.0])
+    sim.execute()
+    want, _ = oracle_mod.sph_execute(recs, [1.0, 2.0, 1.0], 2)
+    assert_bits_equal(sim.downloadParticles(), want, "records")
+    sim.close()
+
+
+def test_quotients_outside_the_fast_range(cuda, pkg, oracle_mod):
+    """Neighbours whose force terms leave the range of the shared-reciprocal
+    quotients (tiny and huge velocities, infinities, NaN, near-coincident
+    particles) get the divisions' results."""
+    recs = pkg.sph_scene_dambreak([1.0, 2.0, 1.0], 4000, 5)
+    rng = np.random.default_rng(4)
+    recs[:, 4:7] = rng.normal(0.0, 1.0, (len(recs), 3)) * 10.0 ** rng.integers(-38, 39, (len(recs), 1))
+    recs[7, 4], recs[99, 5], recs[500, 6] = np.inf, -np.inf, np.nan
+    recs[1000:1010, 0:3] = recs[1000, 0:3] + np.float32(1e-30)
+    recs[2000:2010, 0] = np.nextafter(recs[2000, 0], np.float32(9), dtype=np.float32)
+    recs[2000:2010, 1:3] = recs[2000, 1:3]
+    sim = pkg.SPHSimulator(None, None, 0.08, maxParticles=4000)
+    for warp_max in (-1, 0):
+        sim.warpPerParticle = warp_max
+        sim.upload(recs, [1.0, 2.0, 1.0])
+        sim.execute(substeps=1)
+        want, _ = oracle_mod.sph_execute(recs, [1.0, 2.0, 1.0], 1)
+        got = sim.downloadParticles()
+        nan = np.isnan(want)
+        assert np.array_equal(nan, np.isnan(got))
+        assert_bits_equal(np.where(nan, 0, got), np.where(nan, 0, want), "records")
+    sim.close()
+
+
 def test_posvel_feeds_the_renderer(cuda, pkg):
     import math
     sim = pkg.SPHSimulator(None, None, 0.08)

@@ -4,18 +4,18 @@
 // viscosity forces (sph/force.wgsl), integration with penalty walls
 // (sph/integrate.wgsl) and the posvel copy (sph/copyPosition.wgsl).
 //
-// Per substep (two per execute(), sph.ts:325-355):
+// Per substep (two per execute(), sph.ts:325-355), six launches:
 //   k_sph_bin       cell of every particle (the grid's fixed [-2, 2]^3
-//                   domain plus a sentinel), per-cell counts
-//   k_sph_blocksum, k_sph_scan   exclusive prefix sum of the counts
-//   k_sph_scatter   particle order by cell; each cell's run sorted by
-//                   particle index (k_sph_cellsort)
-//   k_sph_gather    sorted copies of positions and velocities
+//                   domain plus a sentinel), counts per cell and per chunk
+//                   of cells
+//   k_sph_scan      exclusive prefix sum of the counts
+//   k_sph_scatter   particle order by cell
+//   k_sph_place     each cell's run in ascending particle index, with sorted
+//                   copies of positions and velocities
 //   k_sph_density   per sorted slot: density and near density over the
 //                   3x3x3 neighbouring cells (x runs merged, as the shader)
 //   k_sph_force     per sorted slot: pressure, near pressure, viscosity,
-//                   gravity
-//   k_sph_integrate walls, velocity and position update, posvel
+//                   gravity; then walls, velocity and position update, posvel
 //
 // Arithmetic restates the shaders with every f32 operation explicitly
 // rounded (no contraction), in the shaders' operation order.  Two choices
@@ -32,6 +32,7 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/mpm.h"
@@ -75,434 +76,35 @@ __device__ __forceinline__ int cell_number(const Env& e, int xi, int yi, int zi)
                  (unsigned)zi * (unsigned)e.X * (unsigned)e.Y);
 }
 
-__global__ void k_sph_bin(float4* __restrict__ P, float4* __restrict__ V, float4* __restrict__ F,
-                          int n, Env e, int* __restrict__ cell_of, unsigned* __restrict__ count,
-                          unsigned* __restrict__ rank) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float4 p = P[i];
-    int xi, yi, zi;
-    cell_pos(e, p.x, p.y, p.z, xi, yi, zi);
-    const int c = cell_number(e, xi, yi, zi);
-    const bool in = c >= 0 && c < e.total;
-    cell_of[i] = in ? c : -1;
-    if (in) rank[i] = atomicAdd(count + c, 1u);
-    // densities are recomputed this substep; particles outside the grid keep
-    // zero (density.wgsl:58-59) and so a zero force (force.wgsl)
-    p.w = 0.0f;
-    P[i] = p;
-    float4 v = V[i];
-    v.w = 0.0f;
-    V[i] = v;
-    if (!in) F[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+// Where a substep's results go, per particle.
+struct SphOut {
+    float4 *P, *V, *F, *posvel;
+};
+
+__device__ __forceinline__ void write_posvel(float4* __restrict__ posvel, size_t i, const float4& p,
+                                             const float4& v) {
+    posvel[2 * i] = make_float4(p.x, p.y, p.z, 0.0f);
+    posvel[2 * i + 1] = make_float4(v.x, v.y, v.z, 0.0f);
 }
 
-// Exclusive scan of count[0 .. m) into start[0 .. m] in two passes: per-CTA
-// sums of kScan counts, then each CTA scans its own counts after adding the
-// sums of the CTAs before it (at most a few hundred).
-constexpr int kScan = 1024;
-
-__device__ __forceinline__ unsigned block_exclusive(unsigned x, unsigned* s_w, unsigned& total) {
-    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    unsigned v = x;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned y = __shfl_up_sync(0xffffffffu, v, o);
-        if ((int)lane >= o) v += y;
-    }
-    if (lane == 31) s_w[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-        unsigned w = s_w[lane];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned y = __shfl_up_sync(0xffffffffu, w, o);
-            if ((int)lane >= o) w += y;
-        }
-        s_w[lane] = w;
-    }
-    __syncthreads();
-    total = s_w[31];
-    return v - x + (warp ? s_w[warp - 1] : 0u);
-}
-
-__global__ void __launch_bounds__(kScan) k_sph_blocksum(const unsigned* __restrict__ count, int m,
-                                                        unsigned* __restrict__ sums) {
-    __shared__ unsigned s_w[32];
-    const int k = blockIdx.x * kScan + threadIdx.x;
-    unsigned total;
-    block_exclusive(k < m ? count[k] : 0u, s_w, total);
-    if (threadIdx.x == 0) sums[blockIdx.x] = total;
-}
-
-__global__ void __launch_bounds__(kScan) k_sph_scan(const unsigned* __restrict__ count,
-                                                    const unsigned* __restrict__ sums, int m,
-                                                    unsigned* __restrict__ start) {
-    __shared__ unsigned s_w[32];
-    __shared__ unsigned s_pre;
-    // sums of the CTAs before this one
-    unsigned pre = 0;
-    for (int b = threadIdx.x; b < (int)blockIdx.x; b += kScan) pre += sums[b];
-    unsigned tp;
-    block_exclusive(pre, s_w, tp);
-    if (threadIdx.x == 0) s_pre = tp;
-    __syncthreads();
-    const unsigned base = s_pre;
-    const int k = blockIdx.x * kScan + threadIdx.x;
-    const unsigned c = k < m ? count[k] : 0u;
-    unsigned tot;
-    const unsigned ex = block_exclusive(c, s_w, tot);
-    if (k < m) start[k] = base + ex;
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) start[m] = base + tot;
-}
-
-__global__ void k_sph_scatter(const int* __restrict__ cell_of, const unsigned* __restrict__ rank,
-                              const unsigned* __restrict__ start, int n, unsigned* __restrict__ order) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int c = cell_of[i];
-    if (c >= 0) order[start[c] + rank[i]] = (unsigned)i;
-}
-
-// Each cell's run in ascending particle index (insertion sort; runs are
-// short at SPH densities).
-__global__ void k_sph_cellsort(const unsigned* __restrict__ start, int total,
-                               unsigned* __restrict__ order) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= total) return;
-    const unsigned b = start[c], en = start[c + 1];
-    for (unsigned k = b + 1; k < en; ++k) {
-        const unsigned v = order[k];
-        unsigned j = k;
-        while (j > b && order[j - 1] > v) {
-            order[j] = order[j - 1];
-            --j;
-        }
-        order[j] = v;
-    }
-}
-
-__global__ void k_sph_gather(const float4* __restrict__ P, const float4* __restrict__ V,
-                             const unsigned* __restrict__ order, const unsigned* __restrict__ nbin,
-                             float4* __restrict__ SP, float4* __restrict__ SV) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= (int)*nbin) return;
-    const unsigned i = order[s];
-    SP[s] = P[i];
-    SV[s] = V[i];
-}
-
-// density.wgsl:37-47
-__device__ __forceinline__ float density_kernel(const Env& e, float r) {
-    const float dd = sub(e.kr2, mul(r, r));
-    return mul(mul(mul(e.s_density, dd), dd), dd);
-}
-__device__ __forceinline__ float near_density_kernel(const Env& e, float r) {
-    const float d = sub(e.kr, r);
-    return mul(mul(mul(e.s_near, d), d), d);
-}
-
-__device__ __forceinline__ bool in_grid(const Env& e, int xi, int yi, int zi) {
-    return xi < e.X && 0 <= xi && yi < e.Y && 0 <= yi && zi < e.Z && 0 <= zi;
-}
-
-// density.wgsl:58-100, per sorted slot.
-__global__ void k_sph_density(float4* __restrict__ P, float4* __restrict__ V,
-                              float4* __restrict__ SP, float4* __restrict__ SV,
-                              const unsigned* __restrict__ order, const unsigned* __restrict__ start,
-                              Env e) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= (int)start[e.total]) return;
-    const float4 pi = SP[s];
-    int vx, vy, vz;
-    cell_pos(e, pi.x, pi.y, pi.z, vx, vy, vz);
-    float dens = 0.0f, near = 0.0f;
-    if (in_grid(e, vx, vy, vz)) {
-        for (int dz = max(-1, -vz); dz <= min(1, e.Z - vz - 1); ++dz)
-            for (int dy = max(-1, -vy); dy <= min(1, e.Y - vy - 1); ++dy) {
-                const int dxmin = max(-1, -vx), dxmax = min(1, e.X - vx - 1);
-                const int c0 = cell_number(e, vx + dxmin, vy + dy, vz + dz);
-                const int c1 = cell_number(e, vx + dxmax, vy + dy, vz + dz);
-                const unsigned b = start[c0], en = start[c1 + 1];
-                for (unsigned j = b; j < en; ++j) {
-                    const float4 pj = SP[j];
-                    const float dx = sub(pi.x, pj.x), dyv = sub(pi.y, pj.y), dzv = sub(pi.z, pj.z);
-                    const float r2 = add(add(mul(dx, dx), mul(dyv, dyv)), mul(dzv, dzv));
-                    if (r2 < e.kr2) {
-                        dens = add(dens, mul(e.mass, density_kernel(e, __fsqrt_rn(r2))));
-                        near = add(near, mul(e.mass, near_density_kernel(e, __fsqrt_rn(r2))));
-                    }
-                }
-            }
-    }
-    const unsigned i = order[s];
-    SP[s].w = dens;
-    SV[s].w = near;
-    P[i].w = dens;
-    V[i].w = near;
-}
-
-// force.wgsl:37-56
-__device__ __forceinline__ float grad_kernel(const Env& e, float r) {
-    const float d = sub(e.kr, r);
-    return mul(mul(e.s_grad, d), d);
-}
-__device__ __forceinline__ float near_grad_kernel(const Env& e, float r) {
-    const float d = sub(e.kr, r);
-    return mul(mul(e.s_near_grad, d), d);
-}
-__device__ __forceinline__ float lap_kernel(const Env& e, float r) {
-    return mul(e.s_lap, sub(e.kr, r));
-}
-
-// force.wgsl:64-128, per sorted slot.
-__global__ void k_sph_force(const float4* __restrict__ SP, const float4* __restrict__ SV,
-                            const unsigned* __restrict__ order, const unsigned* __restrict__ start,
-                            Env e, float4* __restrict__ F) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= (int)start[e.total]) return;
-    const float4 pi = SP[s], vi = SV[s];
-    const float dens_i = pi.w, near_i = vi.w;
-    float fp[3] = {0.0f, 0.0f, 0.0f}, fv[3] = {0.0f, 0.0f, 0.0f};
-    int vx, vy, vz;
-    cell_pos(e, pi.x, pi.y, pi.z, vx, vy, vz);
-    if (in_grid(e, vx, vy, vz)) {
-        for (int dz = max(-1, -vz); dz <= min(1, e.Z - vz - 1); ++dz)
-            for (int dy = max(-1, -vy); dy <= min(1, e.Y - vy - 1); ++dy) {
-                const int dxmin = max(-1, -vx), dxmax = min(1, e.X - vx - 1);
-                const int c0 = cell_number(e, vx + dxmin, vy + dy, vz + dz);
-                const int c1 = cell_number(e, vx + dxmax, vy + dy, vz + dz);
-                const unsigned b = start[c0], en = start[c1 + 1];
-                for (unsigned j = b; j < en; ++j) {
-                    const float4 pj = SP[j], vj = SV[j];
-                    const float dens_j = pj.w, near_j = vj.w;
-                    const float dx = sub(pi.x, pj.x), dyv = sub(pi.y, pj.y), dzv = sub(pi.z, pj.z);
-                    const float r2 = add(add(mul(dx, dx), mul(dyv, dyv)), mul(dzv, dzv));
-                    if (dens_j == 0.0f || near_j == 0.0f) continue;
-                    if (r2 < e.kr2 && 0.0f < r2) {
-                        const float r = __fsqrt_rn(r2);
-                        const float p_i = mul(e.stiffness, sub(dens_i, e.rest_density));
-                        const float p_j = mul(e.stiffness, sub(dens_j, e.rest_density));
-                        const float np_i = mul(e.near_stiffness, near_i);
-                        const float np_j = mul(e.near_stiffness, near_j);
-                        const float sp = dvd(add(p_i, p_j), 2.0f);
-                        const float nsp = dvd(add(np_i, np_j), 2.0f);
-                        // normalize(pos_j - pos_i)
-                        const float ux = sub(pj.x, pi.x), uy = sub(pj.y, pi.y), uz = sub(pj.z, pi.z);
-                        const float len = __fsqrt_rn(add(add(mul(ux, ux), mul(uy, uy)), mul(uz, uz)));
-                        const float dir[3] = {dvd(ux, len), dvd(uy, len), dvd(uz, len)};
-                        const float g = grad_kernel(e, r), ng = near_grad_kernel(e, r);
-                        const float a = mul(-e.mass, sp), an = mul(-e.mass, nsp);
-                        const float lap = lap_kernel(e, r);
-                        const float rel[3] = {sub(vj.x, vi.x), sub(vj.y, vi.y), sub(vj.z, vi.z)};
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) {
-                            fp[c] = add(fp[c], dvd(mul(mul(a, dir[c]), g), dens_j));
-                            fp[c] = add(fp[c], dvd(mul(mul(an, dir[c]), ng), near_j));
-                            fv[c] = add(fv[c], dvd(mul(mul(e.mass, rel[c]), lap), dens_j));
-                        }
-                    }
-                }
-            }
-    }
-    const float grv[3] = {mul(dens_i, 0.0f), mul(dens_i, -9.8f), mul(dens_i, 0.0f)};
+// The end of force.wgsl:64-128 (gravity), integrate.wgsl:37-64 (penalty walls
+// of the real box, velocity and position) and copyPosition.wgsl:27-37 for
+// particle i: p = position and density, v = velocity and near density.  Done
+// where the forces are summed: the particle is in registers there, and the
+// neighbours' copies (DP, DV) are not what is written.
+__device__ __forceinline__ void finish_particle(const Env& e, float4 p, float4 v,
+                                                const float (&fp)[3], const float (&fv)[3],
+                                                const float* __restrict__ box, const SphOut& out,
+                                                size_t i) {
+    const float dens = p.w;
+    const float grv[3] = {mul(dens, 0.0f), mul(dens, -9.8f), mul(dens, 0.0f)};
     float f[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) f[c] = add(add(fp[c], mul(fv[c], e.viscosity)), grv[c]);
-    F[order[s]] = make_float4(f[0], f[1], f[2], 0.0f);
-}
-
-
-// ---------------------------------------------------------------------------
-// Warp per particle (small particle counts: one thread per particle leaves
-// the SMs with a few warps each, waiting on the neighbour loop).  The lanes
-// compute the neighbour terms of up to kSphChunk neighbours at a time into
-// shared memory, then one lane per accumulator adds them in the neighbours'
-// order, so every sum is the thread kernel's, bit for bit.
-// ---------------------------------------------------------------------------
-constexpr int kSphChunk = 64;
-constexpr int kSphWarps = 8;  // warps (particles) per 256-thread block
-
-// The up to 9 runs of sorted slots (one per (dz, dy) row, x merged) that
-// hold a particle's neighbours, in the thread kernels' visiting order.
-struct NeighbourRows {
-    unsigned b[9], len[9];
-    int n = 0, total = 0;
-};
-
-__device__ __forceinline__ void neighbour_rows(const Env& e, const unsigned* __restrict__ start,
-                                               int vx, int vy, int vz, NeighbourRows& nr) {
-    nr.n = 0;
-    nr.total = 0;
-#pragma unroll
-    for (int r = 0; r < 9; ++r) nr.b[r] = nr.len[r] = 0u;
-    if (!in_grid(e, vx, vy, vz)) return;
-    int r = 0;
-    for (int dz = max(-1, -vz); dz <= min(1, e.Z - vz - 1); ++dz)
-        for (int dy = max(-1, -vy); dy <= min(1, e.Y - vy - 1); ++dy) {
-            const int dxmin = max(-1, -vx), dxmax = min(1, e.X - vx - 1);
-            const int c0 = cell_number(e, vx + dxmin, vy + dy, vz + dz);
-            const int c1 = cell_number(e, vx + dxmax, vy + dy, vz + dz);
-            const unsigned b = start[c0], en = start[c1 + 1];
-#pragma unroll
-            for (int q = 0; q < 9; ++q)
-                if (q == r) {
-                    nr.b[q] = b;
-                    nr.len[q] = en - b;
-                }
-            nr.total += (int)(en - b);
-            ++r;
-        }
-    nr.n = r;
-}
-
-// Sorted slot of the k-th neighbour (k < total).
-__device__ __forceinline__ unsigned neighbour_slot(const NeighbourRows& nr, int k) {
-    unsigned j = 0u, off = 0u;
-    bool found = false;
-#pragma unroll
-    for (int r = 0; r < 9; ++r) {
-        if (!found && (unsigned)k < off + nr.len[r]) {
-            j = nr.b[r] + ((unsigned)k - off);
-            found = true;
-        }
-        off += nr.len[r];
-    }
-    return j;
-}
-
-// density.wgsl:58-100 as k_sph_density, one warp per sorted slot.
-__global__ void __launch_bounds__(32 * kSphWarps)
-    k_sph_density_warp(float4* __restrict__ P, float4* __restrict__ V, float4* __restrict__ SP,
-                       float4* __restrict__ SV, const unsigned* __restrict__ order,
-                       const unsigned* __restrict__ start, Env e) {
-    __shared__ float s_t[kSphWarps][2][kSphChunk];
-    __shared__ unsigned char s_ok[kSphWarps][kSphChunk];
-    const int w = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31u);
-    const int s = (int)blockIdx.x * kSphWarps + w;
-    if (s >= (int)start[e.total]) return;  // uniform per warp
-    const float4 pi = SP[s];
-    int vx, vy, vz;
-    cell_pos(e, pi.x, pi.y, pi.z, vx, vy, vz);
-    NeighbourRows nr;
-    neighbour_rows(e, start, vx, vy, vz, nr);
-    float acc = 0.0f;  // lane 0: density, lane 1: near density
-    for (int base = 0; base < nr.total; base += kSphChunk) {
-        const int m = min(kSphChunk, nr.total - base);
-        for (int q = lane; q < m; q += 32) {
-            const float4 pj = SP[neighbour_slot(nr, base + q)];
-            const float dx = sub(pi.x, pj.x), dyv = sub(pi.y, pj.y), dzv = sub(pi.z, pj.z);
-            const float r2 = add(add(mul(dx, dx), mul(dyv, dyv)), mul(dzv, dzv));
-            const bool ok = r2 < e.kr2;
-            s_ok[w][q] = ok;
-            if (ok) {
-                s_t[w][0][q] = mul(e.mass, density_kernel(e, __fsqrt_rn(r2)));
-                s_t[w][1][q] = mul(e.mass, near_density_kernel(e, __fsqrt_rn(r2)));
-            }
-        }
-        __syncwarp();
-        if (lane < 2)
-            for (int q = 0; q < m; ++q)
-                if (s_ok[w][q]) acc = add(acc, s_t[w][lane][q]);
-        __syncwarp();
-    }
-    const float near = __shfl_sync(0xffffffffu, acc, 1);
-    if (lane == 0) {
-        const unsigned i = order[s];
-        SP[s].w = acc;
-        SV[s].w = near;
-        P[i].w = acc;
-        V[i].w = near;
-    }
-}
-
-// force.wgsl:64-128 as k_sph_force, one warp per sorted slot.
-__global__ void __launch_bounds__(32 * kSphWarps)
-    k_sph_force_warp(const float4* __restrict__ SP, const float4* __restrict__ SV,
-                     const unsigned* __restrict__ order, const unsigned* __restrict__ start,
-                     Env e, float4* __restrict__ F) {
-    __shared__ float s_t[kSphWarps][9][kSphChunk];
-    __shared__ unsigned char s_ok[kSphWarps][kSphChunk];
-    const int w = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31u);
-    const int s = (int)blockIdx.x * kSphWarps + w;
-    if (s >= (int)start[e.total]) return;  // uniform per warp
-    const float4 pi = SP[s], vi = SV[s];
-    const float dens_i = pi.w, near_i = vi.w;
-    int vx, vy, vz;
-    cell_pos(e, pi.x, pi.y, pi.z, vx, vy, vz);
-    NeighbourRows nr;
-    neighbour_rows(e, start, vx, vy, vz, nr);
-    // lanes 0-2: pressure force component c (two terms per neighbour), lanes
-    // 3-5: viscosity force component c
-    float acc = 0.0f;
-    for (int base = 0; base < nr.total; base += kSphChunk) {
-        const int m = min(kSphChunk, nr.total - base);
-        for (int q = lane; q < m; q += 32) {
-            const unsigned j = neighbour_slot(nr, base + q);
-            const float4 pj = SP[j], vj = SV[j];
-            const float dens_j = pj.w, near_j = vj.w;
-            const float dx = sub(pi.x, pj.x), dyv = sub(pi.y, pj.y), dzv = sub(pi.z, pj.z);
-            const float r2 = add(add(mul(dx, dx), mul(dyv, dyv)), mul(dzv, dzv));
-            const bool ok = !(dens_j == 0.0f || near_j == 0.0f) && r2 < e.kr2 && 0.0f < r2;
-            s_ok[w][q] = ok;
-            if (ok) {
-                const float r = __fsqrt_rn(r2);
-                const float p_i = mul(e.stiffness, sub(dens_i, e.rest_density));
-                const float p_j = mul(e.stiffness, sub(dens_j, e.rest_density));
-                const float np_i = mul(e.near_stiffness, near_i);
-                const float np_j = mul(e.near_stiffness, near_j);
-                const float sp = dvd(add(p_i, p_j), 2.0f);
-                const float nsp = dvd(add(np_i, np_j), 2.0f);
-                const float ux = sub(pj.x, pi.x), uy = sub(pj.y, pi.y), uz = sub(pj.z, pi.z);
-                const float len = __fsqrt_rn(add(add(mul(ux, ux), mul(uy, uy)), mul(uz, uz)));
-                const float dir[3] = {dvd(ux, len), dvd(uy, len), dvd(uz, len)};
-                const float g = grad_kernel(e, r), ng = near_grad_kernel(e, r);
-                const float a = mul(-e.mass, sp), an = mul(-e.mass, nsp);
-                const float lap = lap_kernel(e, r);
-                const float rel[3] = {sub(vj.x, vi.x), sub(vj.y, vi.y), sub(vj.z, vi.z)};
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    s_t[w][c][q] = dvd(mul(mul(a, dir[c]), g), dens_j);
-                    s_t[w][3 + c][q] = dvd(mul(mul(an, dir[c]), ng), near_j);
-                    s_t[w][6 + c][q] = dvd(mul(mul(e.mass, rel[c]), lap), dens_j);
-                }
-            }
-        }
-        __syncwarp();
-        if (lane < 3) {
-            for (int q = 0; q < m; ++q)
-                if (s_ok[w][q]) {
-                    acc = add(acc, s_t[w][lane][q]);
-                    acc = add(acc, s_t[w][3 + lane][q]);
-                }
-        } else if (lane < 6) {
-            for (int q = 0; q < m; ++q)
-                if (s_ok[w][q]) acc = add(acc, s_t[w][3 + lane][q]);
-        }
-        __syncwarp();
-    }
-    const float fv = __shfl_down_sync(0xffffffffu, acc, 3);  // lane c gets lane 3 + c's
-    const float grv[3] = {mul(dens_i, 0.0f), mul(dens_i, -9.8f), mul(dens_i, 0.0f)};
-    float f = 0.0f;
-    if (lane < 3) f = add(add(acc, mul(fv, e.viscosity)), grv[lane]);
-    const float f1 = __shfl_sync(0xffffffffu, f, 1), f2 = __shfl_sync(0xffffffffu, f, 2);
-    if (lane == 0) F[order[s]] = make_float4(f, f1, f2, 0.0f);
-}
-
-// integrate.wgsl:37-64 and copyPosition.wgsl:27-37.
-__global__ void k_sph_integrate(float4* __restrict__ P, float4* __restrict__ V,
-                                const float4* __restrict__ F, int n, Env e,
-                                const float* __restrict__ box, float4* __restrict__ posvel) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float rx = box[0], ry = box[1], rz = box[2];
-    float4 p = P[i], v = V[i];
-    const float dens = p.w;
     if (dens != 0.0f) {
-        const float4 f = F[i];
-        float a[3] = {dvd(f.x, dens), dvd(f.y, dens), dvd(f.z, dens)};
+        float a[3] = {dvd(f[0], dens), dvd(f[1], dens), dvd(f[2], dens)};
         const float ws = 8000.0f;
-        const float half[3] = {rx, ry, rz};
+        const float half[3] = {box[0], box[1], box[2]};
         const float pos[3] = {p.x, p.y, p.z};
         float plus[3][3], minus[3][3];  // [axis][component]
 #pragma unroll
@@ -528,13 +130,609 @@ __global__ void k_sph_integrate(float4* __restrict__ P, float4* __restrict__ V,
         p.x = add(p.x, mul(e.dt, v.x));
         p.y = add(p.y, mul(e.dt, v.y));
         p.z = add(p.z, mul(e.dt, v.z));
-        P[i] = p;
-        V[i] = v;
     }
-    if (posvel) {
-        posvel[2 * (size_t)i] = make_float4(p.x, p.y, p.z, 0.0f);
-        posvel[2 * (size_t)i + 1] = make_float4(v.x, v.y, v.z, 0.0f);
+    out.P[i] = p;
+    out.V[i] = v;
+    out.F[i] = make_float4(f[0], f[1], f[2], 0.0f);
+    write_posvel(out.posvel, i, p, v);
+}
+
+// Cells per chunk of the counts' scan, and the chunks the domain can have.
+constexpr int kScan = 1024;
+constexpr int kMaxChunks = 256;  // 62^3 cells: 233
+
+// Cell of every particle with its rank among the cell's arrivals, and the
+// counts per cell and per chunk of cells (through shared memory: the particles
+// of a settled pool share a few dozen chunks).  Particles outside the grid
+// keep zero densities (density.wgsl:58-59) and so a zero force (force.wgsl) and
+// their place; the others' results come from the force kernels.
+__global__ void __launch_bounds__(256)
+    k_sph_bin(SphOut out, int n, Env e, int* __restrict__ cell_of, unsigned* __restrict__ count,
+              unsigned* __restrict__ chunk, unsigned* __restrict__ rank) {
+    __shared__ unsigned s_chunk[kMaxChunks];
+    for (int k = threadIdx.x; k < kMaxChunks; k += 256) s_chunk[k] = 0u;
+    __syncthreads();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < n) {
+        float4 p = out.P[i];
+        int xi, yi, zi;
+        cell_pos(e, p.x, p.y, p.z, xi, yi, zi);
+        const int c = cell_number(e, xi, yi, zi);
+        const bool in = c >= 0 && c < e.total;
+        cell_of[i] = in ? c : -1;
+        if (in) {
+            rank[i] = atomicAdd(count + c, 1u);
+            atomicAdd(&s_chunk[c / kScan], 1u);
+        } else {
+            float4 v = out.V[i];
+            p.w = v.w = 0.0f;
+            out.P[i] = p;
+            out.V[i] = v;
+            out.F[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            write_posvel(out.posvel, i, p, v);
+        }
     }
+    __syncthreads();
+    for (int k = threadIdx.x; k < kMaxChunks; k += 256)
+        if (s_chunk[k]) atomicAdd(chunk + k, s_chunk[k]);
+}
+
+// Exclusive scan of count[0 .. m) into start[0 .. m]: each CTA adds up the
+// chunk counts before its own (at most a few hundred, counted with the cells)
+// and scans its chunk; the counts are left zero for the next binning.
+__device__ __forceinline__ unsigned block_exclusive(unsigned x, unsigned* s_w, unsigned& total) {
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    unsigned v = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, v, o);
+        if ((int)lane >= o) v += y;
+    }
+    if (lane == 31) s_w[warp] = v;
+    __syncthreads();
+    if (warp == 0) {
+        unsigned w = s_w[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned y = __shfl_up_sync(0xffffffffu, w, o);
+            if ((int)lane >= o) w += y;
+        }
+        s_w[lane] = w;
+    }
+    __syncthreads();
+    total = s_w[31];
+    return v - x + (warp ? s_w[warp - 1] : 0u);
+}
+
+__global__ void __launch_bounds__(kScan) k_sph_scan(unsigned* __restrict__ count,
+                                                    const unsigned* __restrict__ chunk, int m,
+                                                    unsigned* __restrict__ start) {
+    __shared__ unsigned s_w[32];
+    const int k = blockIdx.x * kScan + threadIdx.x;
+    const unsigned c = k < m ? count[k] : 0u;
+    unsigned base, tot;
+    block_exclusive(threadIdx.x < blockIdx.x ? chunk[threadIdx.x] : 0u, s_w, base);
+    __syncthreads();  // s_w reused
+    const unsigned ex = block_exclusive(c, s_w, tot);
+    if (k < m) {
+        start[k] = base + ex;
+        if (c) count[k] = 0u;
+    }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) start[m] = base + tot;
+}
+
+__global__ void __launch_bounds__(256)
+    k_sph_scatter(const int* __restrict__ cell_of, const unsigned* __restrict__ rank,
+                  const unsigned* __restrict__ start, int n, unsigned* __restrict__ chunk,
+                  unsigned* __restrict__ arrival) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < kMaxChunks) chunk[i] = 0u;  // for the next binning
+    if (i >= n) return;
+    const int c = cell_of[i];
+    if (c >= 0) arrival[start[c] + rank[i]] = (unsigned)i;
+}
+
+// Each cell's run in ascending particle index: a particle's slot is the
+// cell's first one plus the number of smaller indices in the run (a handful at
+// SPH densities).  One thread per particle, not per cell: most of the domain's
+// cells are empty and a full one's run would be sorted by one thread.
+__global__ void __launch_bounds__(256)
+    k_sph_place(const float4* __restrict__ P, const float4* __restrict__ V,
+                const int* __restrict__ cell_of, const unsigned* __restrict__ start, int total,
+                const unsigned* __restrict__ arrival, unsigned* __restrict__ order,
+                float4* __restrict__ SP, float4* __restrict__ SV) {
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= start[total]) return;
+    const unsigned i = arrival[t];
+    const float4 p = P[i], v = V[i];
+    const int c = cell_of[i];
+    const unsigned b = start[c], en = start[c + 1];
+    unsigned s = b;
+    for (unsigned j = b; j < en; ++j) s += arrival[j] < i ? 1u : 0u;
+    order[s] = i;
+    SP[s] = p;
+    SV[s] = v;
+}
+
+// density.wgsl:37-47
+__device__ __forceinline__ float density_kernel(const Env& e, float r) {
+    const float dd = sub(e.kr2, mul(r, r));
+    return mul(mul(mul(e.s_density, dd), dd), dd);
+}
+__device__ __forceinline__ float near_density_kernel(const Env& e, float r) {
+    const float d = sub(e.kr, r);
+    return mul(mul(mul(e.s_near, d), d), d);
+}
+
+__device__ __forceinline__ bool in_grid(const Env& e, int xi, int yi, int zi) {
+    return xi < e.X && 0 <= xi && yi < e.Y && 0 <= yi && zi < e.Z && 0 <= zi;
+}
+
+// force.wgsl:37-56
+__device__ __forceinline__ float grad_kernel(const Env& e, float r) {
+    const float d = sub(e.kr, r);
+    return mul(mul(e.s_grad, d), d);
+}
+__device__ __forceinline__ float near_grad_kernel(const Env& e, float r) {
+    const float d = sub(e.kr, r);
+    return mul(mul(e.s_near_grad, d), d);
+}
+__device__ __forceinline__ float lap_kernel(const Env& e, float r) {
+    return mul(e.s_lap, sub(e.kr, r));
+}
+
+// Squared distance, in the shaders' order.
+__device__ __forceinline__ float dist2(const float4& a, const float4& b) {
+    const float dx = sub(a.x, b.x), dy = sub(a.y, b.y), dz = sub(a.z, b.z);
+    return add(add(mul(dx, dx), mul(dy, dy)), mul(dz, dz));
+}
+
+// a / b for several a and one b, correctly rounded, from y = RN(1 / b): a
+// first quotient, one Newton correction that brings it to within an ulp, and
+// Markstein's final one, which rounds correctly because the remainder
+// fma(-b, q, a) is exact (P. Markstein, IBM J. Res. Dev. 34, 1990).  Five
+// operations instead of a division.  Holds for quotients in [kQuotMin,
+// kQuotMax] when b lies in [2^-20, 2^40]: no intermediate leaves the normal
+// range.  rcp_for_quotients(b) is NaN for other b, so that every quotient fails
+// the range test; infinities give NaN too.
+constexpr float kQuotMin = 1.0e-20f, kQuotMax = 1.0e20f;
+
+__device__ __forceinline__ float rcp_for_quotients(float b) {
+    return b >= 0x1p-20f && b <= 0x1p40f ? __frcp_rn(b) : __int_as_float(0x7fc00000);
+}
+
+__device__ __forceinline__ float quot(float a, float b, float y) {
+    float q = mul(a, y);
+    q = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+    return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+}
+
+// The larger of two, NaN when one is.
+__device__ __forceinline__ float fmax_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+// The terms that neighbour j (position pj with its density, velocity vj with
+// its near density, reciprocals rj of the two) adds to the forces of particle
+// i: t[0..2] pressure, t[3..5] near pressure, t[6..8] viscosity
+// (force.wgsl:96-120).  A listed particle that is none (the particle itself,
+// one without a density) adds nothing: +0, which leaves a sum that started at
+// +0 as it is.
+__device__ __forceinline__ void force_terms(const Env& e, const float4& pi, const float4& vi,
+                                            const float4& pj, const float4& vj, const float2& rj,
+                                            float (&t)[9]) {
+    const float dens_j = pj.w, near_j = vj.w;
+    const float r2 = dist2(pi, pj);
+    if (dens_j == 0.0f || near_j == 0.0f || !(0.0f < r2)) {
+#pragma unroll
+        for (int q = 0; q < 9; ++q) t[q] = 0.0f;
+        return;
+    }
+    // normalize(pos_j - pos_i): the same length as the distance (the
+    // differences are exact negatives)
+    const float r = __fsqrt_rn(r2);
+    const float p_i = mul(e.stiffness, sub(pi.w, e.rest_density));
+    const float p_j = mul(e.stiffness, sub(dens_j, e.rest_density));
+    const float np_i = mul(e.near_stiffness, vi.w);
+    const float np_j = mul(e.near_stiffness, near_j);
+    const float sp = mul(add(p_i, p_j), 0.5f);     // / 2, exactly
+    const float nsp = mul(add(np_i, np_j), 0.5f);
+    const float u[3] = {sub(pj.x, pi.x), sub(pj.y, pi.y), sub(pj.z, pi.z)};
+    const float g = grad_kernel(e, r), ng = near_grad_kernel(e, r);
+    const float a = mul(-e.mass, sp), an = mul(-e.mass, nsp);
+    const float lap = lap_kernel(e, r);
+    const float rel[3] = {sub(vj.x, vi.x), sub(vj.y, vi.y), sub(vj.z, vi.z)};
+    const float rr = rcp_for_quotients(r);
+    float lo = kQuotMax, hi = kQuotMin;
+    auto seen = [&](float q) {
+        lo = fminf(lo, fabsf(q));
+        hi = fmax_nan(hi, fabsf(q));
+        return q;
+    };
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const float dir = seen(quot(u[c], r, rr));
+        t[c] = seen(quot(mul(mul(a, dir), g), dens_j, rj.x));
+        t[3 + c] = seen(quot(mul(mul(an, dir), ng), near_j, rj.y));
+        t[6 + c] = seen(quot(mul(mul(e.mass, rel[c]), lap), dens_j, rj.x));
+    }
+    if (lo >= kQuotMin && hi <= kQuotMax) return;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const float dir = dvd(u[c], r);
+        t[c] = dvd(mul(mul(a, dir), g), dens_j);
+        t[3 + c] = dvd(mul(mul(an, dir), ng), near_j);
+        t[6 + c] = dvd(mul(mul(e.mass, rel[c]), lap), dens_j);
+    }
+}
+
+// Sorted slots [b, en) of row r (dz = r / 3 - 1, dy = r % 3 - 1, the three
+// cells along x merged) of the cells around (vx, vy, vz), in the shaders'
+// visiting order for r = 0 .. 8; empty where the row leaves the grid.
+__device__ __forceinline__ void neighbour_row(const Env& e, const unsigned* __restrict__ start,
+                                              int vx, int vy, int vz, int r, unsigned& b,
+                                              unsigned& en) {
+    const int z = vz + r / 3 - 1, y = vy + r % 3 - 1;
+    b = en = 0u;
+    if (z < 0 || z >= e.Z || y < 0 || y >= e.Y) return;
+    b = start[cell_number(e, max(vx - 1, 0), y, z)];
+    en = start[cell_number(e, min(vx + 1, e.X - 1), y, z) + 1];
+}
+
+// ---------------------------------------------------------------------------
+// Density and forces.  Bound by instruction issue (densities, 70-78 % of the
+// issue slots) and by the latency of the neighbours' gathers (forces).  Of the
+// candidates in the 27 cells around a particle one in five is a neighbour, and
+// a neighbour's terms cost 2 (density) to 8 times (force) what testing a
+// candidate does.  With the terms computed where a candidate passes, some lane
+// of a warp passes at nearly every candidate and the others wait (20 % of the
+// lanes active in the force).  So the density kernels first collect the
+// neighbours that pass, in visiting order, and then compute their terms with
+// all lanes busy; they leave the list in memory for the force kernels.  Every
+// sum adds its terms in the visiting order, so all variants give the same
+// bits.  Per two-substep frame of settled pools, with one warp (10,000
+// particles) or one thread per particle testing and computing as it goes, and
+// now (the sort's launches included): 10,000 particles 169 -> 55 us, 40,000
+// 308 -> 96 us, 400,000 1830 -> 730 us.
+// ---------------------------------------------------------------------------
+
+// Neighbours listed per particle (a settled pool has 25-60, its bottom up to
+// 100; a particle with more walks its rows again for the force: with 64, the
+// bottom's did, 400,000 particles 1165 instead of 758 us).  Entry k of sorted
+// particle s is nbr[k * stride + s], so that neighbouring particles' entries
+// share sectors.  No lists are kept for capacities above kListedMax, where
+// they would take over 4 GB.
+constexpr int kNeighbours = 128;
+constexpr int kListedMax = 1 << 23;
+
+struct NeighbourLists {
+    unsigned* nbr;   // null: no lists
+    int* n;          // neighbours of each sorted particle, listed or not
+    size_t stride;
+    __device__ __forceinline__ bool listed(int count) const { return nbr && count <= kNeighbours; }
+    __device__ __forceinline__ void put(int s, int k, unsigned j) const {
+        if (nbr && k < kNeighbours) nbr[(size_t)k * stride + s] = j;
+    }
+    __device__ __forceinline__ unsigned get(int s, int k) const { return nbr[(size_t)k * stride + s]; }
+};
+
+// G lanes per particle: the lanes test G candidates of a row at a time and a
+// ballot gives the ones that pass their places in the list; the lanes compute
+// the listed neighbours' terms into shared memory and one lane per accumulator
+// adds them in list order.  All control flow is uniform over the warp, whose
+// 32 / G particles go through their rows together.
+constexpr int kGroupBlock = 256;
+
+template <int G>
+struct Group {
+    static constexpr int kParticles = kGroupBlock / G;  // particles per block
+    static constexpr unsigned kMask = G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u;
+    int p, lane;      // particle of the block, lane of the group
+    unsigned shift;   // the group's first lane in the warp
+    int m = 0;        // listed neighbours of this round
+    int taken = 0;    // and of the rounds before it
+    __device__ Group()
+        : p((int)threadIdx.x / G), lane((int)threadIdx.x % G), shift(threadIdx.x & 31u & ~(unsigned)(G - 1)) {}
+    // This lane's place in the list when its candidate passes (else -1).
+    // Every lane of the warp calls it.
+    __device__ __forceinline__ int append(bool pass) {
+        const unsigned hits = (__ballot_sync(0xffffffffu, pass) >> shift) & kMask;
+        const int at = pass ? m + __popc(hits & ((1u << lane) - 1u)) : -1;
+        m += __popc(hits);
+        return at;
+    }
+};
+
+// Walks the candidates of this group's particle (none unless `in`), Q per lane
+// at a time with all their positions loaded first: put(place, j, r2) for those
+// within the kernel radius, take() when the round's list of L has no room for
+// G * Q more and at the end.
+template <int G, int Q, int L, class Put, class Take>
+__device__ __forceinline__ void walk_neighbours(const Env& e, const unsigned* __restrict__ start,
+                                                const float4* __restrict__ pos, int pos_stride,
+                                                const float4& pi, bool in, Group<G>& g, Put&& put,
+                                                Take&& take) {
+    static_assert(L >= G * Q, "a batch fits an empty list");
+    int vx, vy, vz;
+    cell_pos(e, pi.x, pi.y, pi.z, vx, vy, vz);
+    in = in && in_grid(e, vx, vy, vz);
+#pragma unroll 3
+    for (int row = 0; row < 9; ++row) {
+        unsigned b = 0u, en = 0u;
+        if (in) neighbour_row(e, start, vx, vy, vz, row, b, en);
+        for (unsigned j0 = b; __any_sync(0xffffffffu, j0 < en); j0 += G * Q) {
+            if (__any_sync(0xffffffffu, g.m > L - G * Q)) take();
+            float r2[Q];
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                const unsigned j = j0 + (unsigned)(q * G + g.lane);
+                r2[q] = e.kr2;
+                if (j < en) r2[q] = dist2(pi, pos[(size_t)j * pos_stride]);
+            }
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                const int at = g.append(r2[q] < e.kr2);
+                if (at >= 0) put(at, j0 + (unsigned)(q * G + g.lane), r2[q]);
+            }
+        }
+    }
+    take();
+}
+
+__device__ __forceinline__ void write_density(float4* __restrict__ D, float2* __restrict__ DR,
+                                              const float4* __restrict__ SV, int s,
+                                              const float4& pi, float dens, float near) {
+    const float4 v = SV[s];
+    D[2 * (size_t)s] = make_float4(pi.x, pi.y, pi.z, dens);
+    D[2 * (size_t)s + 1] = make_float4(v.x, v.y, v.z, near);
+    DR[s] = make_float2(rcp_for_quotients(dens), rcp_for_quotients(near));
+}
+
+// density.wgsl:58-100, per sorted slot.
+template <int G>
+__global__ void __launch_bounds__(kGroupBlock)
+    k_sph_density(const float4* __restrict__ SP, const float4* __restrict__ SV,
+                  float4* __restrict__ D, float2* __restrict__ DR, NeighbourLists nl,
+                  const unsigned* __restrict__ start, Env e) {
+    using Gr = Group<G>;
+    constexpr int kList = 64;
+    __shared__ float2 s_t[Gr::kParticles][kList];  // r2 and slot of the listed, then their two terms
+    const int nbin = (int)start[e.total];
+    if ((int)blockIdx.x * Gr::kParticles >= nbin) return;
+    Gr g;
+    const int s = (int)blockIdx.x * Gr::kParticles + g.p;
+    const bool active = s < nbin;
+    const float4 pi = active ? SP[s] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float2* t = s_t[g.p];
+    float acc = 0.0f;  // lane 0: density, lane 1: near density
+    walk_neighbours<G, 32 / G, kList>(
+        e, start, SP, 1, pi, active, g,
+        [&](int at, unsigned j, float r2) { t[at] = make_float2(r2, __uint_as_float(j)); },
+        [&]() {
+            __syncwarp();
+            for (int k = g.lane; k < g.m; k += G) {
+                const float2 u = t[k];
+                const float r = __fsqrt_rn(u.x);
+                t[k] = make_float2(mul(e.mass, density_kernel(e, r)),
+                                   mul(e.mass, near_density_kernel(e, r)));
+                nl.put(s, g.taken + k, __float_as_uint(u.y));
+            }
+            __syncwarp();
+            if (g.lane < 2) {
+                const float* u = &t[0].x + g.lane;
+#pragma unroll 4
+                for (int k = 0; k < g.m; ++k) acc = add(acc, u[2 * k]);
+            }
+            g.taken += g.m;
+            g.m = 0;
+            __syncwarp();
+        });
+    const float near = __shfl_sync(0xffffffffu, acc, (int)g.shift + 1);
+    if (active && g.lane == 0) {
+        write_density(D, DR, SV, s, pi, acc, near);
+        nl.n[s] = g.taken;
+    }
+}
+
+// The same with one thread per particle, for many particles: a test costs no
+// ballot and the terms no trip through shared memory (290 instead of 614
+// warp instructions per particle), at a few warps per scheduler.  The list of a
+// round is the thread's own column in shared memory; 32 entries, because more
+// would take the L1 cache that the candidates' positions live in (64 entries
+// and one candidate loaded at a time: 264 instead of 177 us at 400,000
+// particles).  The lanes of a warp (neighbouring
+// sorted slots) take their terms together, when some lane's list is full and at
+// the end: a lane that took its terms alone would hold up the other 31.
+constexpr int kThreadBlock = 128;
+constexpr int kThreadList = 32;
+constexpr int kThreadStep = 4;  // candidates loaded at a time
+
+__global__ void __launch_bounds__(kThreadBlock)
+    k_sph_density_thread(const float4* __restrict__ SP, const float4* __restrict__ SV,
+                         float4* __restrict__ D, float2* __restrict__ DR, NeighbourLists nl,
+                         const unsigned* __restrict__ start, Env e) {
+    __shared__ unsigned s_j[kThreadList][kThreadBlock];
+    const int nbin = (int)start[e.total];
+    const int s = blockIdx.x * kThreadBlock + threadIdx.x;
+    if ((s & ~31) >= nbin) return;  // uniform per warp
+    const bool active = s < nbin;
+    const float4 pi = active ? SP[s] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    int vx, vy, vz;
+    cell_pos(e, pi.x, pi.y, pi.z, vx, vy, vz);
+    const bool in = active && in_grid(e, vx, vy, vz);
+    float dens = 0.0f, near = 0.0f;
+    int m = 0, taken = 0;
+    auto take = [&]() {
+#pragma unroll 2
+        for (int k = 0; k < m; ++k) {
+            const unsigned j = s_j[k][threadIdx.x];
+            nl.put(s, taken + k, j);
+            const float r = __fsqrt_rn(dist2(pi, SP[j]));
+            dens = add(dens, mul(e.mass, density_kernel(e, r)));
+            near = add(near, mul(e.mass, near_density_kernel(e, r)));
+        }
+        taken += m;
+        m = 0;
+        __syncwarp();
+    };
+    for (int row = 0; row < 9; ++row) {
+        unsigned b = 0u, en = 0u;
+        if (in) neighbour_row(e, start, vx, vy, vz, row, b, en);
+        while (__any_sync(0xffffffffu, b < en)) {
+            if (__any_sync(0xffffffffu, m > kThreadList - kThreadStep)) take();
+            float4 p[kThreadStep];
+#pragma unroll
+            for (int q = 0; q < kThreadStep; ++q) p[q] = SP[min(b + q, (unsigned)nbin - 1u)];
+#pragma unroll
+            for (int q = 0; q < kThreadStep; ++q)
+                if (b + q < en && dist2(pi, p[q]) < e.kr2) s_j[m++][threadIdx.x] = b + q;
+            b += kThreadStep;
+        }
+    }
+    take();
+    if (!active) return;
+    write_density(D, DR, SV, s, pi, dens, near);
+    nl.n[s] = taken;
+}
+
+// force.wgsl:64-128 and the integration, per sorted slot.  D: position and
+// density, velocity and near density of each sorted particle (one 32-byte
+// sector, for the gathers); DR: the densities' reciprocals.
+template <int G>
+__global__ void __launch_bounds__(kGroupBlock)
+    k_sph_force(const float4* __restrict__ D, const float2* __restrict__ DR,
+                NeighbourLists nl, const unsigned* __restrict__ order,
+                const unsigned* __restrict__ start, Env e, const float* __restrict__ box,
+                SphOut out) {
+    using Gr = Group<G>;
+    constexpr int kList = 32;  // 36 KB for G = 8: four blocks an SM, as the registers allow
+    __shared__ unsigned s_j[Gr::kParticles][kList];
+    __shared__ float s_t[Gr::kParticles][9 * kList];
+    const int nbin = (int)start[e.total];
+    if ((int)blockIdx.x * Gr::kParticles >= nbin) return;
+    Gr g;
+    const int s = (int)blockIdx.x * Gr::kParticles + g.p;
+    const bool active = s < nbin;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const int total = active ? nl.n[s] : 0;
+    const float4 pi = active ? D[2 * (size_t)s] : zero, vi = active ? D[2 * (size_t)s + 1] : zero;
+    float* t = s_t[g.p];
+    // lanes 0-2: pressure force component c (two terms per neighbour), lanes
+    // 3-5: viscosity force component c
+    float acc = 0.0f;
+    auto put_terms = [&](int k, unsigned j) {
+        float q[9];
+        force_terms(e, pi, vi, D[2 * (size_t)j], D[2 * (size_t)j + 1], DR[j], q);
+#pragma unroll
+        for (int c = 0; c < 9; ++c) t[9 * k + c] = q[c];
+    };
+    auto add_terms = [&](int m) {
+        if (g.lane < 6) {
+            const bool pressure = g.lane < 3;
+            const float* u = t + (pressure ? g.lane : g.lane + 3);
+#pragma unroll 4
+            for (int k = 0; k < m; ++k) {
+                acc = add(acc, u[9 * k]);
+                if (pressure) acc = add(acc, u[9 * k + 3]);
+            }
+        }
+    };
+    if (__all_sync(0xffffffffu, nl.listed(total))) {
+        // entries of a round are loaded while the round before it computes
+        constexpr int kPer = kList / G;
+        unsigned j[kPer];
+        auto load = [&](int base) {
+#pragma unroll
+            for (int q = 0; q < kPer; ++q) {
+                const int k = base + q * G + g.lane;
+                j[q] = k < total ? nl.get(s, k) : 0u;
+            }
+        };
+        load(0);
+        for (int base = 0; __any_sync(0xffffffffu, base < total); base += kList) {
+            unsigned now[kPer];
+#pragma unroll
+            for (int q = 0; q < kPer; ++q) now[q] = j[q];
+            load(base + kList);
+            const int m = min(total - base, kList);
+#pragma unroll
+            for (int q = 0; q < kPer; ++q)
+                if (q * G + g.lane < m) put_terms(q * G + g.lane, now[q]);
+            __syncwarp();
+            add_terms(m);
+            __syncwarp();
+        }
+    } else {
+        unsigned* list = s_j[g.p];
+        walk_neighbours<G, 1, kList>(
+            e, start, D, 2, pi, active, g, [&](int at, unsigned j, float) { list[at] = j; },
+            [&]() {
+                __syncwarp();
+                for (int k = g.lane; k < g.m; k += G) put_terms(k, list[k]);
+                __syncwarp();
+                add_terms(g.m);
+                g.m = 0;
+                __syncwarp();
+            });
+    }
+    float fp[3], fv[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        fp[c] = __shfl_sync(0xffffffffu, acc, (int)g.shift + c);
+        fv[c] = __shfl_sync(0xffffffffu, acc, (int)g.shift + 3 + c);
+    }
+    if (active && g.lane == 0) finish_particle(e, pi, vi, fp, fv, box, out, order[s]);
+}
+
+
+// One thread per particle: the next neighbour's record is gathered while this
+// one's terms are computed.
+__global__ void __launch_bounds__(kThreadBlock)
+    k_sph_force_thread(const float4* __restrict__ D, const float2* __restrict__ DR,
+                       NeighbourLists nl, const unsigned* __restrict__ order,
+                       const unsigned* __restrict__ start, Env e, const float* __restrict__ box,
+                       SphOut out) {
+    const int s = blockIdx.x * kThreadBlock + threadIdx.x;
+    if (s >= (int)start[e.total]) return;
+    const int total = nl.n[s];
+    const float4 pi = D[2 * (size_t)s], vi = D[2 * (size_t)s + 1];
+    float fp[3] = {0.0f, 0.0f, 0.0f}, fv[3] = {0.0f, 0.0f, 0.0f};
+    auto add_terms = [&](const float4& pj, const float4& vj, const float2& rj) {
+        float t[9];
+        force_terms(e, pi, vi, pj, vj, rj, t);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            fp[c] = add(add(fp[c], t[c]), t[3 + c]);
+            fv[c] = add(fv[c], t[6 + c]);
+        }
+    };
+    if (nl.listed(total)) {
+        unsigned j = total > 0 ? nl.get(s, 0) : 0u, j2 = total > 1 ? nl.get(s, 1) : 0u;
+        float4 pj = D[2 * (size_t)j], vj = D[2 * (size_t)j + 1];
+        float2 rj = DR[j];
+        for (int k = 0; k < total; ++k) {
+            const float4 pc = pj, vc = vj;
+            const float2 rc = rj;
+            pj = D[2 * (size_t)j2];
+            vj = D[2 * (size_t)j2 + 1];
+            rj = DR[j2];
+            j2 = k + 2 < total ? nl.get(s, k + 2) : 0u;
+            add_terms(pc, vc, rc);
+        }
+    } else {
+        int vx, vy, vz;
+        cell_pos(e, pi.x, pi.y, pi.z, vx, vy, vz);
+        for (int row = 0; row < 9 && in_grid(e, vx, vy, vz); ++row) {
+            unsigned b, en;
+            neighbour_row(e, start, vx, vy, vz, row, b, en);
+            for (unsigned j = b; j < en; ++j)
+                if (dist2(pi, D[2 * (size_t)j]) < e.kr2)
+                    add_terms(D[2 * (size_t)j], D[2 * (size_t)j + 1], DR[j]);
+        }
+    }
+    finish_particle(e, pi, vi, fp, fv, box, out, order[s]);
 }
 
 int fail(int code, const std::string& msg) {
@@ -561,10 +759,18 @@ struct SplitMix64 {
 
 }  // namespace
 
-// Default for mpm_sph::warp_max: below it a warp per particle, above it a
-// thread per particle fills the GPU with fewer instructions.  Measured per
-// 2-substep frame (warp / thread): 20k particles 0.285 / 0.359 ms, 40k
-// 0.599 / 0.499 ms.
+// Which density and force kernels run at n particles.  Frames in us, settled
+// pools (16 lanes / 8 lanes / 8 lanes for the densities and a thread for the
+// forces / a thread for both): 8,000 particles 51 / 54 / 66 / 101, 12,000 60 /
+// 60 / 69 / 109, 24,000 87 / 83 / 81 / 119, 100,000 268 / 222 / 182 / 190,
+// 130,000 330 / 281 / 229 / 225, 400,000 - / 1097 / 836 / 758: the fewer the
+// particles, the more lanes it takes to hide a particle's chain of loads, and
+// the more of them the fewer instructions decide.
+constexpr int kSph16Max = 12000;
+constexpr int kSphLanesMax = 22000;
+constexpr int kSphDensity8Max = 130000;
+// Default of mpm_sph::warp_max: particle counts above it run no group of lanes
+// for the forces, whatever the limits above allow.
 constexpr int kSphWarpMaxDefault = 32768;
 
 struct mpm_sph {
@@ -574,18 +780,24 @@ struct mpm_sph {
     float render_diameter = 0.0f;
     float real_half[3] = {0, 0, 0};
     Env e{};
-    float4 *P = nullptr, *V = nullptr, *F = nullptr, *SP = nullptr, *SV = nullptr;
+    char* slab = nullptr;  // the allocation that holds the buffers below, but posvel
+    float4 *P = nullptr, *V = nullptr, *F = nullptr;      // by particle
+    float4 *SP = nullptr, *SV = nullptr;                  // sorted
+    float4* D = nullptr;                                  // sorted, with the densities
+    float2* DR = nullptr;                                 // their reciprocals
+    NeighbourLists nl{};
     float4* posvel = nullptr;
     bool posvel_owned = false;
     int* cell_of = nullptr;
     unsigned *count = nullptr, *start = nullptr, *rank = nullptr, *order = nullptr;
-    unsigned* sums = nullptr;  // per-CTA count sums of the scan
+    unsigned* arrival = nullptr;  // particles by cell, in the order they were counted
+    unsigned* chunk = nullptr;    // counts per kScan cells
     // the real box as the kernels read it (a device uniform, so that a
     // captured frame graph survives changeBoxSize)
     float* box_d = nullptr;
     float box_uploaded[3] = {NAN, NAN, NAN};
     bool graph = true;
-    int warp_max = kSphWarpMaxDefault;  // particle counts up to this run a warp per particle
+    int warp_max = kSphWarpMaxDefault;  // see above
     struct FrameGraph {
         int substeps, n;
         cudaGraphExec_t exec;
@@ -602,11 +814,8 @@ void drop_graphs(mpm_sph* s) {
 
 void free_sph(mpm_sph* s) {
     drop_graphs(s);
-    cudaFree(s->box_d);
-    cudaFree(s->P); cudaFree(s->V); cudaFree(s->F); cudaFree(s->SP); cudaFree(s->SV);
+    cudaFree(s->slab);
     if (s->posvel_owned) cudaFree(s->posvel);
-    cudaFree(s->cell_of); cudaFree(s->count); cudaFree(s->start); cudaFree(s->rank);
-    cudaFree(s->order); cudaFree(s->sums);
     delete s;
 }
 
@@ -667,9 +876,40 @@ int mpm_sph_create(int max_particles, float render_diameter, void* posvel_device
     s->render_diameter = render_diameter;
     s->e = make_env();
     const size_t np = (size_t)(max_particles > 0 ? max_particles : 1);
-    cudaError_t err = cudaSuccess;
-    float4** bufs[5] = {&s->P, &s->V, &s->F, &s->SP, &s->SV};
-    for (int b = 0; b < 5 && err == cudaSuccess; ++b) err = cudaMalloc(bufs[b], sizeof(float4) * np);
+    const size_t cells = (size_t)s->e.total + 1;
+    // one allocation for all of the solver's buffers (an allocation costs as
+    // much as a frame), each at a 256-byte boundary; twice through the list:
+    // once for the size, once for the places
+    size_t bytes = 0;
+    auto place = [&](auto& ptr, size_t count) {
+        if (s->slab) ptr = reinterpret_cast<std::remove_reference_t<decltype(ptr)>>(s->slab + bytes);
+        bytes += (sizeof(*ptr) * count + 255) / 256 * 256;
+    };
+    auto place_all = [&]() {
+        bytes = 0;
+        for (float4** b : {&s->P, &s->V, &s->F, &s->SP, &s->SV}) place(*b, np);
+        place(s->D, 2 * np);
+        place(s->DR, np);
+        place(s->cell_of, np);
+        place(s->rank, np);
+        place(s->order, np);
+        place(s->arrival, np);
+        place(s->nl.n, np);
+        place(s->count, cells);
+        place(s->chunk, kMaxChunks);
+        place(s->start, cells);
+        place(s->box_d, 3);
+        if (np <= kListedMax) place(s->nl.nbr, kNeighbours * np);
+    };
+    s->nl.stride = np;
+    place_all();
+    cudaError_t err = cudaMalloc(&s->slab, bytes);
+    if (err == cudaSuccess) {
+        place_all();
+        // zero between substeps: the scan and the scatter clear what they have read
+        err = cudaMemset(s->count, 0, 4 * cells);
+        if (err == cudaSuccess) err = cudaMemset(s->chunk, 0, 4 * kMaxChunks);
+    }
     if (err == cudaSuccess) {
         if (posvel_device) {
             s->posvel = static_cast<float4*>(posvel_device);
@@ -678,13 +918,6 @@ int mpm_sph_create(int max_particles, float render_diameter, void* posvel_device
             s->posvel_owned = true;
         }
     }
-    if (err == cudaSuccess) err = cudaMalloc(&s->cell_of, 4 * np);
-    if (err == cudaSuccess) err = cudaMalloc(&s->rank, 4 * np);
-    if (err == cudaSuccess) err = cudaMalloc(&s->order, 4 * np);
-    if (err == cudaSuccess) err = cudaMalloc(&s->count, 4 * ((size_t)s->e.total + 1));
-    if (err == cudaSuccess) err = cudaMalloc(&s->start, 4 * ((size_t)s->e.total + 1));
-    if (err == cudaSuccess) err = cudaMalloc(&s->sums, 4 * ((size_t)s->e.total / kScan + 2));
-    if (err == cudaSuccess) err = cudaMalloc(&s->box_d, sizeof(float) * 3);
     if (err != cudaSuccess) {
         const int rc = cuda_fail(err, "mpm_sph_create");
         free_sph(s);
@@ -770,32 +1003,56 @@ int mpm_sph_set_real_box(mpm_sph* s, const float real_half[3]) {
 
 namespace {
 
+// G lanes (or one thread) per particle.
+template <int G>
+void launch_density(mpm_sph* s, cudaStream_t st) {
+    if constexpr (G == 1) {
+        k_sph_density_thread<<<(s->n + kThreadBlock - 1) / kThreadBlock, kThreadBlock, 0, st>>>(
+            s->SP, s->SV, s->D, s->DR, s->nl, s->start, s->e);
+    } else {
+        const int gb = (s->n + Group<G>::kParticles - 1) / Group<G>::kParticles;
+        k_sph_density<G><<<gb, kGroupBlock, 0, st>>>(s->SP, s->SV, s->D, s->DR, s->nl, s->start, s->e);
+    }
+}
+
+template <int G>
+void launch_force(mpm_sph* s, const SphOut& out, cudaStream_t st) {
+    if constexpr (G == 1) {
+        k_sph_force_thread<<<(s->n + kThreadBlock - 1) / kThreadBlock, kThreadBlock, 0, st>>>(
+            s->D, s->DR, s->nl, s->order, s->start, s->e, s->box_d, out);
+    } else {
+        const int gb = (s->n + Group<G>::kParticles - 1) / Group<G>::kParticles;
+        k_sph_force<G><<<gb, kGroupBlock, 0, st>>>(s->D, s->DR, s->nl, s->order, s->start, s->e,
+                                                   s->box_d, out);
+    }
+}
+
 void enqueue_substeps(mpm_sph* s, int substeps, cudaStream_t st) {
     const int n = s->n;
     const Env& e = s->e;
-    const int pb = (n + 255) / 256, cb = (e.total + 255) / 256;
+    const SphOut out{s->P, s->V, s->F, s->posvel};
+    const int pb = (n + 255) / 256;
+    const int chunks = (e.total + kScan - 1) / kScan;
     for (int k = 0; k < substeps; ++k) {
-        cudaMemsetAsync(s->count, 0, 4 * ((size_t)e.total + 1), st);
-        k_sph_bin<<<pb, 256, 0, st>>>(s->P, s->V, s->F, n, e, s->cell_of, s->count, s->rank);
-        const int sb = (e.total + kScan - 1) / kScan;
-        k_sph_blocksum<<<sb, kScan, 0, st>>>(s->count, e.total, s->sums);
-        k_sph_scan<<<sb, kScan, 0, st>>>(s->count, s->sums, e.total, s->start);
-        k_sph_scatter<<<pb, 256, 0, st>>>(s->cell_of, s->rank, s->start, n, s->order);
-        k_sph_cellsort<<<cb, 256, 0, st>>>(s->start, e.total, s->order);
+        k_sph_bin<<<pb, 256, 0, st>>>(out, n, e, s->cell_of, s->count, s->chunk, s->rank);
+        k_sph_scan<<<chunks, kScan, 0, st>>>(s->count, s->chunk, e.total, s->start);
+        k_sph_scatter<<<pb, 256, 0, st>>>(s->cell_of, s->rank, s->start, n, s->chunk, s->arrival);
         // sorted slots: start[total] of them (read on the device); launched
         // over n, the most there can be
-        k_sph_gather<<<pb, 256, 0, st>>>(s->P, s->V, s->order, s->start + e.total, s->SP, s->SV);
-        if (n <= s->warp_max) {  // one warp per particle
-            const int wb = (n + kSphWarps - 1) / kSphWarps;
-            k_sph_density_warp<<<wb, 32 * kSphWarps, 0, st>>>(s->P, s->V, s->SP, s->SV, s->order,
-                                                               s->start, e);
-            k_sph_force_warp<<<wb, 32 * kSphWarps, 0, st>>>(s->SP, s->SV, s->order, s->start, e,
-                                                             s->F);
+        k_sph_place<<<pb, 256, 0, st>>>(s->P, s->V, s->cell_of, s->start, e.total, s->arrival,
+                                        s->order, s->SP, s->SV);
+        const bool lanes = n <= s->warp_max && n <= kSphLanesMax;
+        if (lanes && n <= kSph16Max) {
+            launch_density<16>(s, st);
+            launch_force<16>(s, out, st);
+        } else if (lanes) {
+            launch_density<8>(s, st);
+            launch_force<8>(s, out, st);
         } else {
-            k_sph_density<<<pb, 256, 0, st>>>(s->P, s->V, s->SP, s->SV, s->order, s->start, e);
-            k_sph_force<<<pb, 256, 0, st>>>(s->SP, s->SV, s->order, s->start, e, s->F);
+            if (n <= kSphDensity8Max) launch_density<8>(s, st);
+            else launch_density<1>(s, st);
+            launch_force<1>(s, out, st);
         }
-        k_sph_integrate<<<pb, 256, 0, st>>>(s->P, s->V, s->F, n, e, s->box_d, s->posvel);
     }
 }
 

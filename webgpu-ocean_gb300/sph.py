@@ -60,8 +60,9 @@ class SPHSimulator:
 
     @property
     def warpPerParticle(self) -> int:
-        """Particle counts up to this run density and forces one warp per
-        particle (default 32768; 0: never; -1 to set: the default)."""
+        """Particle counts up to this may run the forces with several lanes of
+        a warp per particle, and do where that is the faster way (default
+        32768; 0: never; -1 to set: the default).  Results are the same."""
         return _check(self._lib.mpm_sph_get_warp_per_particle(self._handle), "warpPerParticle")
 
     @warpPerParticle.setter
