@@ -194,3 +194,73 @@ def test_sphere_mode_matches_restatement(cuda, pkg, oracle_mod):
     assert (want["depth"] < 1).mean() > 0.03
     r.close()
     sim.close()
+
+
+def splat_both(pkg, oracle_mod, pv, u, W, H, n=None, spheres=True):
+    """Splats through the two public modes: fluid thickness and depth reach
+    the images through filters, so the sphere view checks every pixel's winner
+    and the fluid view the thickness sums."""
+    import torch
+    n = len(pv) if n is None else n
+    dev = torch.from_numpy(np.ascontiguousarray(pv, dtype=np.float32)).cuda()
+    r = pkg.FluidRenderer(W, H, RADIUS, FOV)
+    r.execute(dev, n, u, sphereRenderFl=True)
+    want = oracle_mod.sphere(pv[:n], uniforms_f32(u), W, H)
+    for k in ("color", "color8", "depth"):
+        same_bits(r.download(k), want[k], f"sphere {k}")
+    if not spheres:
+        r.execute(dev, n, u)
+        want = oracle_mod.render(pv[:n], uniforms_f32(u), W, H, RADIUS, FOV, default_env_from(pkg))
+        for k in ("depth", "thickness", "color", "color8"):
+            same_bits(r.download(k), want[k], k)
+    r.close()
+    return want
+
+
+def pool(n, box, seed):
+    rng = np.random.default_rng(seed)
+    pv = np.zeros((n, 8), np.float32)
+    pv[:, 0:3] = rng.random((n, 3)) * np.array(box)
+    pv[:, 4:7] = rng.normal(0.0, 0.5, (n, 3))
+    return pv
+
+
+@pytest.mark.parametrize("n,W,H,dist,size", [
+    (1, 33, 31, 20.0, 1.2), (9999, 64, 64, 40.0, 1.2), (10000, 65, 63, 40.0, 1.2),
+    (39999, 130, 97, 45.0, 1.2), (40000, 96, 33, 45.0, 1.2),   # either side of the item sizes
+    (3000, 200, 150, 12.0, 1.2),     # the camera inside the pool: billboards over many tiles
+    (300, 320, 256, 25.0, 12.0),     # billboards of 100 pixels: none binned
+    (20000, 128, 96, 60.0, 0.01),    # billboards below a pixel
+    (500, 1, 400, 40.0, 1.2), (500, 400, 1, 40.0, 1.2),
+])
+def test_splats_by_tile(cuda, pkg, oracle_mod, n, W, H, dist, size):
+    pv = pool(n, (20.0, 8.0, 24.0), n)
+    pv[:min(50, n // 4), 0:3] = pv[n // 2, 0:3]  # equal depths: the first drawn wins
+    u = pkg.camera_uniforms(W, H, dist, [10.0, 4.0, 12.0], FOV, size)
+    splat_both(pkg, oracle_mod, pv, u, W, H, spheres=False)
+
+
+def test_splats_of_odd_particles_and_cameras(cuda, pkg, oracle_mod):
+    """Positions that are not ordinary numbers, and projections that are not
+    the application's (skewed clip z and w, mirrored axes)."""
+    pv = pool(2000, (20.0, 8.0, 24.0), 3)
+    pv[3:9, 0:3] = [[np.nan, 1, 1], [np.inf, 1, 1], [1, -np.inf, 1], [1e30, 1, 1], [1, 1e38, 1], [-1e20, 1e20, 1e20]]
+    W, H = 150, 110
+    u = pkg.camera_uniforms(W, H, 40.0, [10.0, 4.0, 12.0], FOV, 1.2)
+    splat_both(pkg, oracle_mod, pv, u, W, H, spheres=False)
+    for at, value in ((2, 0.01), (6, -0.02), (3, 0.001), (15, 0.5), (0, None), (5, None), (14, 0.1)):
+        v = pkg.camera_uniforms(W, H, 40.0, [10.0, 4.0, 12.0], FOV, 1.2)
+        v.projection_matrix[at] = -v.projection_matrix[at] if value is None else value
+        splat_both(pkg, oracle_mod, pv, v, W, H)
+
+
+def test_splats_in_rounds_and_without_tiles(cuda, pkg, oracle_mod):
+    """More particles than one round bins, and an image of more tiles than
+    are counted (8,193 columns of tiles)."""
+    pv = pool((1 << 20) + 77, (20.0, 8.0, 24.0), 5)
+    u = pkg.camera_uniforms(60, 45, 50.0, [10.0, 4.0, 12.0], FOV, 1.2)
+    splat_both(pkg, oracle_mod, pv, u, 60, 45)
+    W, H = 32 * 8192 + 5, 2
+    pv = pool(300, (20.0, 8.0, 24.0), 6)
+    u = pkg.camera_uniforms(64, 48, 40.0, [10.0, 4.0, 12.0], FOV, 1.2)
+    splat_both(pkg, oracle_mod, pv, u, W, H)
