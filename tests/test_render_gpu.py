@@ -264,3 +264,24 @@ def test_splats_in_rounds_and_without_tiles(cuda, pkg, oracle_mod):
     pv = pool(300, (20.0, 8.0, 24.0), 6)
     u = pkg.camera_uniforms(64, 48, 40.0, [10.0, 4.0, 12.0], FOV, 1.2)
     splat_both(pkg, oracle_mod, pv, u, W, H)
+
+
+@pytest.mark.parametrize("W,H,radius,dist", [
+    (255, 33, 0.6, 40.0), (257, 31, 0.6, 40.0), (256, 32, 0.6, 8.0),  # filters up to the widest, 100
+    (63, 7, 0.6, 60.0), (65, 9, 0.6, 60.0),
+    (130, 100, 0.5, 40.0), (130, 100, 0.31, 30.0),  # the divisor no power of two
+    (130, 100, 1e-5, 40.0), (130, 100, 2e3, 40.0),  # and out of the shared reciprocal's range
+])
+def test_filters(cuda, pkg, oracle_mod, W, H, radius, dist):
+    """The fluid view's filters at sizes around a block's pixels, from narrow
+    to the widest, and every way of dividing by the depth sigma."""
+    import torch
+    pv = pool(6000, (20.0, 8.0, 24.0), W)
+    u = pkg.camera_uniforms(W, H, dist, [10.0, 4.0, 12.0], FOV, 1.2)
+    dev = torch.from_numpy(pv).cuda()
+    r = pkg.FluidRenderer(W, H, radius, FOV)
+    r.execute(dev, len(pv), u)
+    want = oracle_mod.render(pv, uniforms_f32(u), W, H, radius, FOV, default_env_from(pkg))
+    for k in ("depth", "thickness", "color", "color8"):
+        same_bits(r.download(k), want[k], k)
+    r.close()

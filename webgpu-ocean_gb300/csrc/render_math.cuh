@@ -29,14 +29,8 @@ __device__ __forceinline__ float dvd(float a, float b) { return __fdiv_rn(a, b);
 // 2^k for k in [-126, 127], exactly.
 __device__ __forceinline__ float pow2i(int k) { return __int_as_float((k + 127) << 23); }
 
-__device__ __forceinline__ float exp_r(float x) {
-    if (x != x) return x;
-    if (x > 88.8f) return __int_as_float(0x7f800000);
-    if (x < -104.0f) return 0.0f;
-    const float kf = rintf(mul(x, 1.44269502f));  // nearest integer of x / ln2
-    const int k = (int)kf;
-    const float r = sub(sub(x, mul(kf, 0.693145751953125f)), mul(kf, 1.42860677e-6f));
-    // Taylor series of exp(r), Horner form
+// Taylor series of exp(r) to degree 8, |r| <= ln2 / 2, Horner form.
+__device__ __forceinline__ float exp_series(float r) {
     float p = 2.48015873e-5f;                 // 1/8!
     p = add(mul(p, r), 1.98412698e-4f);       // 1/7!
     p = add(mul(p, r), 1.38888889e-3f);       // 1/6!
@@ -46,6 +40,17 @@ __device__ __forceinline__ float exp_r(float x) {
     p = add(mul(p, r), 0.5f);
     p = add(mul(p, r), 1.0f);
     p = add(mul(p, r), 1.0f);
+    return p;
+}
+
+__device__ __forceinline__ float exp_r(float x) {
+    if (x != x) return x;
+    if (x > 88.8f) return __int_as_float(0x7f800000);
+    if (x < -104.0f) return 0.0f;
+    const float kf = rintf(mul(x, 1.44269502f));  // nearest integer of x / ln2
+    const int k = (int)kf;
+    const float r = sub(sub(x, mul(kf, 0.693145751953125f)), mul(kf, 1.42860677e-6f));
+    const float p = exp_series(r);
     // p * 2^k in two exact power-of-two steps (k in [-150, 128])
     const int k1 = k / 2, k2 = k - k1;
     return mul(mul(p, pow2i(k1)), pow2i(k2));
