@@ -395,3 +395,32 @@ def test_backward_matches_cpu_tape_adjoint(cuda, pkg, oracle_mod, T, every):
         assert err < 2e-4, f"{name}: max error {err:.2e} of the gradient's scale {scale:.3e}"
     for j, name in enumerate(("stiffness", "viscosity")):
         assert abs(pg[0, j] - pwant[j]) <= 2e-4 * abs(pwant[j]) + 1e-12, (name, pg[0, j], pwant[j])
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 63, 64, 65, 1000])
+def test_fp64_tape_stencils(cuda, pkg, oracle_mod, n):
+    """The FP64 forward at counts around its warps and blocks, with particles
+    at the walls (stencils that alias or leave the grid), outside the box, and
+    too far out for integer cell coordinates, against the FP64 oracle.  Both
+    sum in FP64 in their own order; the states are read as f32, so they agree
+    within an f32 rounding."""
+    rng = np.random.default_rng(n)
+    box = [14.0, 11.0, 17.0]
+    recs = np.zeros((n, 20), np.float32)
+    recs[:, 0:3] = rng.uniform(3.0, 8.0, (n, 3))
+    recs[:, 4:7] = rng.normal(0.0, 0.3, (n, 3))
+    for c in (8, 12, 16):
+        recs[:, c:c + 3] = rng.normal(0.0, 0.1, (n, 3))
+    odd = np.array([[0.3, 5, 5], [13.6, 5, 5], [5, 0.1, 5], [5, 10.7, 5], [5, 5, 16.9], [-2.5, 5, 5],
+                    [5, 5, 40.0], [5.0e8, 5, 5], [-3.0e9, 5, 5], [5, 1.0e30, 5]], np.float32)
+    m = min(len(odd), n // 3)
+    recs[:m, 0:3] = odd[:m]
+    T = 3
+    adj = pkg.MLSMPMAdjoint([pkg.scene_desc(n, box)], T, 1, tape="fp64")
+    adj.forward(recs, T)
+    st = oracle_mod.records_to_state64(recs)
+    for t in range(1, T + 1):
+        st = oracle_mod.run64(st, oracle_mod.Params64.make(box), 1)
+        got = oracle_mod.records_to_state64(adj.state(t))
+        np.testing.assert_allclose(got, st, rtol=2.0 ** -23, atol=1e-9, err_msg=f"substep {t}")
+    adj.close()

@@ -808,91 +808,182 @@ __device__ __forceinline__ int d2i_sat(double x) {
     return (int)x;
 }
 
-__device__ __forceinline__ int flat64(double cx, double cy, double cz, int Y, int Z) {
-    const unsigned a = (unsigned)d2i_sat(cx) * (unsigned)Y * (unsigned)Z;
-    const unsigned b = (unsigned)d2i_sat(cy) * (unsigned)Z;
-    return (int)(a + b + (unsigned)d2i_sat(cz));
-}
+// A particle's stencil in FP64: per axis the cell coordinates, weights and
+// distances (cell centre - x) of its three cells.  FP64 instructions are what
+// the kernels below are short of (1/64 of the f32 rate), so the coordinates are
+// integers wherever floor(x) is one without saturating.
+struct Sten64 {
+    int c[3][3];
+    double w[3][3], d[3][3];  // [axis][g]
+};
 
-__device__ __forceinline__ void weights64(const double* x, double ci[3], double w[3][3]) {
+__device__ __forceinline__ void make_sten64(const double (&x)[3], Sten64& s) {
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        ci[a] = floor(x[a]);
-        const double d = x[a] - (ci[a] + 0.5);
-        w[a][0] = 0.5 * (0.5 - d) * (0.5 - d);
-        w[a][1] = 0.75 - d * d;
-        w[a][2] = 0.5 * (0.5 + d) * (0.5 + d);
+        double ci;
+        if ((__double2hiint(x[a]) & 0x7fffffff) < 0x41d00000) {  // |x| < 2^30
+            const int i = __double2int_rd(x[a]);
+            ci = (double)i;
+#pragma unroll
+            for (int g = 0; g < 3; ++g) s.c[a][g] = i + g - 1;
+        } else {
+            ci = floor(x[a]);
+#pragma unroll
+            for (int g = 0; g < 3; ++g) s.c[a][g] = d2i_sat(ci + g - 1.0);
+        }
+        const double d = x[a] - (ci + 0.5), lo = 0.5 - d, hi = 0.5 + d;
+        s.w[a][0] = 0.5 * lo * lo;
+        s.w[a][1] = fma(-d, d, 0.75);
+        s.w[a][2] = 0.5 * hi * hi;
+        s.d[a][0] = -1.0 - d;
+        s.d[a][1] = -d;
+        s.d[a][2] = 1.0 - d;
     }
 }
 
-// One thread per particle: these kernels are bound by FP64 arithmetic, so
-// splitting a particle's stencil over lanes (which repeats the weights)
-// only adds work.
-__global__ void __launch_bounds__(kThreads)
-    k64_p2g(const double* __restrict__ S, double4* __restrict__ G,
-            const AdjScene* __restrict__ scenes, const int* __restrict__ pscene, int n, int stage) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// Flat index of a stencil cell (wrapping, as the solver's), -1 outside the grid.
+__device__ __forceinline__ int index64(const Sten64& s, int gx, int gy, int gz, const SimConsts& k) {
+    const unsigned i = ((unsigned)s.c[0][gx] * (unsigned)k.Y + (unsigned)s.c[1][gy]) * (unsigned)k.Z +
+                       (unsigned)s.c[2][gz];
+    return i < (unsigned)k.grid_count ? (int)i : -1;
+}
+
+// One thread per particle: bound by FP64 instructions, which lanes sharing a
+// particle would repeat (four lanes, a component each: 700 instead of 270 FP64
+// instructions for stage 1).  The products and sums are factored along the
+// axes and fused.  Small blocks, so that 32,768 particles spread evenly.
+// ncu at 32,768 particles: p2g stages 81 -> 27 and 34 us, g2p 82 -> 31 us;
+// with four lanes per particle 54, 74 and 60.
+constexpr int kThreads64 = 64;
+
+// Adds a stencil cell's contributions of the warp's 32 particles to the grid.
+// A lane holds up to four components of its particle's cell (idx, -1: none);
+// the additions are made by four lanes per cell, from shared memory, so that a
+// warp instruction covers the sectors of eight cells instead of a component of
+// 32.  Every lane calls it, with the buffer alternating.
+template <int N>
+struct CellAdds {
+    double (*val)[4];  // [32] of this warp and buffer
+    int* idx;
+    __device__ __forceinline__ void operator()(double* __restrict__ grid0, int lb_idx,
+                                               const double (&v)[N]) const {
+        const int lane = (int)(threadIdx.x & 31u);
+        idx[lane] = lb_idx;
+#pragma unroll
+        for (int r = 0; r < N; ++r) val[lane][r] = v[r];
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int p = 8 * q + (lane >> 2), r = lane & 3;
+            const int at = idx[p];
+            if (at >= 0 && r < N) atomicAdd(grid0 + 4 * (size_t)at + r, val[p][r]);
+        }
+    }
+};
+
+__global__ void __launch_bounds__(kThreads64)
+    k64_p2g1(const double* __restrict__ S, double4* __restrict__ G,
+             const AdjScene* __restrict__ scenes, const int* __restrict__ pscene, int n) {
+    __shared__ __align__(16) double s_val[kThreads64 / 32][2][32][4];
+    __shared__ int s_idx[kThreads64 / 32][2][32];
+    const int t = blockIdx.x * kThreads64 + threadIdx.x, warp = threadIdx.x >> 5;
+    const bool active = t < n;
+    const int i = active ? t : n - 1;
     const AdjScene& sc = scenes[pscene[i]];
     const SimConsts& k = sc.k;
-    double* grid = reinterpret_cast<double*>(G + sc.lbase);
     const double* P = S + (size_t)kRec64 * i;
-    double x[3] = {P[0], P[1], P[2]};
-    double ci[3], w[3][3];
-    weights64(x, ci, w);
-    double T[3][3];  // stage 2: [row][col]
-    if (stage == 2) {
-        double rho = 0.0;
+    Sten64 st;
+    make_sten64({P[0], P[1], P[2]}, st);
+    int buf = 0;
 #pragma unroll
-        for (int gx = 0; gx < 3; ++gx)
+    for (int gx = 0; gx < 3; ++gx) {
+        double qx[3];  // v + C d, column by column
 #pragma unroll
-            for (int gy = 0; gy < 3; ++gy)
+        for (int r = 0; r < 3; ++r) qx[r] = fma(P[6 + r], st.d[0][gx], P[3 + r]);
 #pragma unroll
-                for (int gz = 0; gz < 3; ++gz) {
-                    const double wt = w[0][gx] * w[1][gy] * w[2][gz];
-                    const int idx = flat64(ci[0] + gx - 1.0, ci[1] + gy - 1.0, ci[2] + gz - 1.0,
-                                           k.Y, k.Z);
-                    if ((unsigned)idx >= (unsigned)k.grid_count) continue;
-                    rho += grid[4 * (size_t)idx + 3] * wt;
-                }
-        const double V = 1.0 / rho;
-        const double rr = rho / (double)k.rest_density;
-        const double pterm = (double)k.stiffness * (rr * rr * rr * rr * rr - 1.0);
-        const double pres = pterm > 0.0 ? pterm : 0.0;
-        for (int a = 0; a < 3; ++a)
-            for (int b = 0; b < 3; ++b) {
-                const double strain = P[6 + 3 * b + a] + P[6 + 3 * a + b];
-                const double sig = (a == b ? -pres : 0.0) + (double)k.dynamic_viscosity * strain;
-                T[a][b] = -V * 4.0 * sig * (double)k.dt;
+        for (int gy = 0; gy < 3; ++gy) {
+            double qxy[3];
+#pragma unroll
+            for (int r = 0; r < 3; ++r) qxy[r] = fma(P[9 + r], st.d[1][gy], qx[r]);
+            const double wxy = st.w[0][gx] * st.w[1][gy];
+#pragma unroll
+            for (int gz = 0; gz < 3; ++gz) {
+                const int idx = active ? index64(st, gx, gy, gz, k) : -1;
+                const double wt = wxy * st.w[2][gz];
+                double v[4];
+#pragma unroll
+                for (int r = 0; r < 3; ++r) v[r] = wt * fma(P[12 + r], st.d[2][gz], qxy[r]);
+                v[3] = wt;
+                CellAdds<4>{s_val[warp][buf], s_idx[warp][buf]}(reinterpret_cast<double*>(G),
+                                                                idx < 0 ? -1 : sc.lbase + idx, v);
+                buf ^= 1;
             }
+        }
     }
+}
+
+__global__ void __launch_bounds__(kThreads64)
+    k64_p2g2(const double* __restrict__ S, double4* __restrict__ G,
+             const AdjScene* __restrict__ scenes, const int* __restrict__ pscene, int n) {
+    __shared__ __align__(16) double s_val[kThreads64 / 32][2][32][4];
+    __shared__ int s_idx[kThreads64 / 32][2][32];
+    const int t = blockIdx.x * kThreads64 + threadIdx.x, warp = threadIdx.x >> 5;
+    const bool active = t < n;
+    const int i = active ? t : n - 1;
+    const AdjScene& sc = scenes[pscene[i]];
+    const SimConsts& k = sc.k;
+    const double* grid = reinterpret_cast<const double*>(G + sc.lbase);
+    const double* P = S + (size_t)kRec64 * i;
+    Sten64 st;
+    make_sten64({P[0], P[1], P[2]}, st);
+    double rho = 0.0;
+#pragma unroll
+    for (int gx = 0; gx < 3; ++gx) {
+        double slab = 0.0;
+#pragma unroll
+        for (int gy = 0; gy < 3; ++gy) {
+            double row = 0.0;
+#pragma unroll
+            for (int gz = 0; gz < 3; ++gz) {
+                const int idx = index64(st, gx, gy, gz, k);
+                if (idx >= 0) row = fma(grid[4 * (size_t)idx + 3], st.w[2][gz], row);
+            }
+            slab = fma(row, st.w[1][gy], slab);
+        }
+        rho = fma(slab, st.w[0][gx], rho);
+    }
+    const double V = 1.0 / rho;
+    const double rr = rho / (double)k.rest_density, r2 = rr * rr;
+    const double pterm = (double)k.stiffness * (r2 * r2 * rr - 1.0);
+    const double pres = pterm > 0.0 ? pterm : 0.0;
+    const double beta = -4.0 * V * (double)k.dt, mu = (double)k.dynamic_viscosity;
+    double T[3][3];  // [row][col], symmetric
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b <= a; ++b)
+            T[a][b] = T[b][a] = beta * fma(mu, P[6 + 3 * b + a] + P[6 + 3 * a + b], a == b ? -pres : 0.0);
+    int buf = 0;
 #pragma unroll
     for (int gx = 0; gx < 3; ++gx)
 #pragma unroll
-        for (int gy = 0; gy < 3; ++gy)
+        for (int gy = 0; gy < 3; ++gy) {
+            double qxy[3];
+#pragma unroll
+            for (int r = 0; r < 3; ++r) qxy[r] = fma(T[r][1], st.d[1][gy], T[r][0] * st.d[0][gx]);
+            const double wxy = st.w[0][gx] * st.w[1][gy];
 #pragma unroll
             for (int gz = 0; gz < 3; ++gz) {
-                const double wt = w[0][gx] * w[1][gy] * w[2][gz];
-                const double c[3] = {ci[0] + gx - 1.0, ci[1] + gy - 1.0, ci[2] + gz - 1.0};
-                double d[3];
+                const int idx = active ? index64(st, gx, gy, gz, k) : -1;
+                const double wt = wxy * st.w[2][gz];
+                double v[3];
 #pragma unroll
-                for (int a = 0; a < 3; ++a) d[a] = (c[a] + 0.5) - x[a];
-                const int idx = flat64(c[0], c[1], c[2], k.Y, k.Z);
-                if ((unsigned)idx >= (unsigned)k.grid_count) continue;
-                double* cell = grid + 4 * (size_t)idx;
-                if (stage == 1) {
-#pragma unroll
-                    for (int r = 0; r < 3; ++r) {
-                        const double q = P[6 + r] * d[0] + P[9 + r] * d[1] + P[12 + r] * d[2];
-                        atomicAdd(cell + r, wt * (P[3 + r] + q));
-                    }
-                    atomicAdd(cell + 3, wt);
-                } else {
-#pragma unroll
-                    for (int r = 0; r < 3; ++r)
-                        atomicAdd(cell + r, wt * (T[r][0] * d[0] + T[r][1] * d[1] + T[r][2] * d[2]));
-                }
+                for (int r = 0; r < 3; ++r) v[r] = wt * fma(T[r][2], st.d[2][gz], qxy[r]);
+                CellAdds<3>{s_val[warp][buf], s_idx[warp][buf]}(reinterpret_cast<double*>(G),
+                                                                idx < 0 ? -1 : sc.lbase + idx, v);
+                buf ^= 1;
             }
+        }
 }
 
 __global__ void __launch_bounds__(kThreads)
@@ -900,6 +991,8 @@ __global__ void __launch_bounds__(kThreads)
                int ncells) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= ncells) return;
+    double4 c = G[j];
+    if (!(c.w > 0.0)) return;
     int lo = 0, hi = nscenes - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
@@ -907,8 +1000,6 @@ __global__ void __launch_bounds__(kThreads)
         else hi = mid - 1;
     }
     const SimConsts& k = scenes[lo].k;
-    double4 c = G[j];
-    if (!(c.w > 0.0)) return;
     const int id = j - scenes[lo].lbase;
     const int xyz[3] = {(id / k.Z) / k.Y, (id / k.Z) % k.Y, id % k.Z};
     double v[3] = {c.x, c.y, c.z};
@@ -925,68 +1016,78 @@ __global__ void __launch_bounds__(kThreads)
     G[j] = c;
 }
 
-__global__ void __launch_bounds__(kThreads)
+// Sums along z, then y, then x.
+__global__ void __launch_bounds__(kThreads64)
     k64_g2p(const double* __restrict__ S, const double4* __restrict__ G, double* __restrict__ Sout,
             const AdjScene* __restrict__ scenes, const int* __restrict__ pscene, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blockIdx.x * kThreads64 + threadIdx.x;
     if (i >= n) return;
     const AdjScene& sc = scenes[pscene[i]];
     const SimConsts& k = sc.k;
-    const double4* grid = G + sc.lbase;
+    const double2* grid = reinterpret_cast<const double2*>(G + sc.lbase);
     const double* P = S + (size_t)kRec64 * i;
     double* Q = Sout + (size_t)kRec64 * i;
     const double x[3] = {P[0], P[1], P[2]};
-    double ci[3], w[3][3];
-    weights64(x, ci, w);
-    double acc[12] = {};  // v (3), then B[c][r] at 3 + 3c + r
+    Sten64 st;
+    make_sten64(x, st);
+    double wd[3][3];  // w d per axis
 #pragma unroll
-    for (int gx = 0; gx < 3; ++gx)
+    for (int a = 0; a < 3; ++a)
 #pragma unroll
-        for (int gy = 0; gy < 3; ++gy)
+        for (int g = 0; g < 3; ++g) wd[a][g] = st.w[a][g] * st.d[a][g];
+    // sums of w u and w u d, u the cells' velocity
+    double v[3] = {}, bx[3] = {}, by[3] = {}, bz[3] = {};
+#pragma unroll
+    for (int gx = 0; gx < 3; ++gx) {
+        double v1[3] = {}, by1[3] = {}, bz1[3] = {};
+#pragma unroll
+        for (int gy = 0; gy < 3; ++gy) {
+            double v2[3] = {}, bz2[3] = {};
 #pragma unroll
             for (int gz = 0; gz < 3; ++gz) {
-                const double wt = w[0][gx] * w[1][gy] * w[2][gz];
-                const double c[3] = {ci[0] + gx - 1.0, ci[1] + gy - 1.0, ci[2] + gz - 1.0};
-                double d[3];
-#pragma unroll
-                for (int a = 0; a < 3; ++a) d[a] = (c[a] + 0.5) - x[a];
-                const int idx = flat64(c[0], c[1], c[2], k.Y, k.Z);
-                double gv[3] = {0.0, 0.0, 0.0};
-                if ((unsigned)idx < (unsigned)k.grid_count) {
-                    const double4 cc = grid[idx];
-                    gv[0] = cc.x; gv[1] = cc.y; gv[2] = cc.z;
-                }
+                const int idx = index64(st, gx, gy, gz, k);
+                if (idx < 0) continue;
+                const double2 a = grid[2 * (size_t)idx];
+                const double u[3] = {a.x, a.y, grid[2 * (size_t)idx + 1].x};
 #pragma unroll
                 for (int r = 0; r < 3; ++r) {
-                    const double wv = gv[r] * wt;
-#pragma unroll
-                    for (int q = 0; q < 3; ++q) acc[3 + 3 * q + r] += wv * d[q];
-                    acc[r] += wv;
+                    v2[r] = fma(st.w[2][gz], u[r], v2[r]);
+                    bz2[r] = fma(wd[2][gz], u[r], bz2[r]);
                 }
+            }
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                v1[r] = fma(st.w[1][gy], v2[r], v1[r]);
+                by1[r] = fma(wd[1][gy], v2[r], by1[r]);
+                bz1[r] = fma(st.w[1][gy], bz2[r], bz1[r]);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            v[r] = fma(st.w[0][gx], v1[r], v[r]);
+            bx[r] = fma(wd[0][gx], v1[r], bx[r]);
+            by[r] = fma(st.w[0][gx], by1[r], by[r]);
+            bz[r] = fma(st.w[0][gx], bz1[r], bz[r]);
+        }
     }
-    const double v[3] = {acc[0], acc[1], acc[2]};
+    const double dt = (double)k.dt;
 #pragma unroll
-    for (int q = 0; q < 3; ++q)
-#pragma unroll
-        for (int r = 0; r < 3; ++r) Q[6 + 3 * q + r] = acc[3 + 3 * q + r] * 4.0;
-    double xo[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        double xx = x[a] + v[a] * (double)k.dt;
-        const double hw = (double)k.real_box[a] - 2.0;
+    for (int r = 0; r < 3; ++r) {
+        Q[6 + r] = 4.0 * bx[r];
+        Q[9 + r] = 4.0 * by[r];
+        Q[12 + r] = 4.0 * bz[r];
+        const double real = (double)k.real_box[r];
+        double xx = x[r] + v[r] * dt;
+        const double hw = real - 2.0;
         xx = xx < 1.0 ? 1.0 : xx;
         xx = xx > hw ? hw : xx;
-        xo[a] = xx;
-        Q[a] = xx;
-    }
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const double xn = xo[a] + v[a] * (double)k.dt * 3.0;
-        const double wmax = (double)k.real_box[a] - 4.0;
-        double va = v[a];
+        Q[r] = xx;
+        const double xn = xx + v[r] * dt * 3.0;
+        const double wmax = real - 4.0;
+        double va = v[r];
         if (xn < 3.0) va += 0.3 * (3.0 - xn);
         if (xn > wmax) va += 0.3 * (wmax - xn);
-        Q[3 + a] = va;
+        Q[3 + r] = va;
     }
     Q[15] = 0.0;
 }
@@ -1055,11 +1156,11 @@ void launch_substep64(const double* S, double4* G, double* Sout, const AdjScene*
                       int nscenes, const int* pscene, int n, int ncells, cudaStream_t st) {
     cudaMemsetAsync(G, 0, sizeof(double4) * (size_t)ncells, st);
     if (n > 0) {
-        k64_p2g<<<blocks(n), kThreads, 0, st>>>(S, G, scenes, pscene, n, 1);
-        k64_p2g<<<blocks(n), kThreads, 0, st>>>(S, G, scenes, pscene, n, 2);
+        k64_p2g1<<<(n + kThreads64 - 1) / kThreads64, kThreads64, 0, st>>>(S, G, scenes, pscene, n);
+        k64_p2g2<<<(n + kThreads64 - 1) / kThreads64, kThreads64, 0, st>>>(S, G, scenes, pscene, n);
     }
     k64_update<<<blocks(ncells), kThreads, 0, st>>>(G, scenes, nscenes, ncells);
-    if (n > 0) k64_g2p<<<blocks(n), kThreads, 0, st>>>(S, G, Sout, scenes, pscene, n);
+    if (n > 0) k64_g2p<<<(n + kThreads64 - 1) / kThreads64, kThreads64, 0, st>>>(S, G, Sout, scenes, pscene, n);
 }
 
 void launch_records_to_rec64(const float* rec, double* S, int n, cudaStream_t st) {
