@@ -424,3 +424,44 @@ def test_fp64_tape_stencils(cuda, pkg, oracle_mod, n):
         got = oracle_mod.records_to_state64(adj.state(t))
         np.testing.assert_allclose(got, st, rtol=2.0 ** -23, atol=1e-9, err_msg=f"substep {t}")
     adj.close()
+
+
+@pytest.mark.parametrize("fm", [1.0e7, 3.0e5 + 1.0, 2.0 ** 21, 2.0 ** -19, 1.2345e6])
+def test_fixed_point_decode_on_the_tape(cuda, pkg, fm):
+    """The backward decodes the fixed-point tape by a shared reciprocal unless
+    a scene's multiplier is out of its range; then every scene divides.  The
+    particles are so far apart that no two share a cell (nothing depends on the
+    order of the atomics), so a scene's gradients are the same bits either way,
+    also when the multiplier changes between two backwards."""
+    i = np.arange(512)
+    recs = np.zeros((512, 20), np.float32)
+    rng = np.random.default_rng(7)
+    recs[:, 0:3] = 5.0 + 4.0 * np.stack([i // 64, i // 8 % 8, i % 8], axis=1) + rng.random((512, 3)) * 0.9
+    recs[:, 4:7] = rng.normal(0.0, 0.1, (512, 3))
+    box, T = [40.0, 40.0, 40.0], 2
+    seed = np.zeros((513, 20), np.float32)
+    seed[:, 0:3] = rng.normal(0.0, 1.0, (513, 3))
+
+    def gradient(adj, rec):
+        adj.forward(rec, T)
+        grad, _ = adj.backward({T: seed[:len(rec)]})
+        return grad[:512]
+
+    one = pkg.scene_desc(512, box, fixed_point_multiplier=fm)
+    adj = pkg.MLSMPMAdjoint([one], T, T, tape="fixed")
+    want = gradient(adj, recs)
+    adj.close()
+    if fm > 1:  # below, every mass truncates to 0 and the gradients are NaN
+        assert np.isfinite(want).all() and np.abs(want).max() > 0
+    lone = np.zeros((1, 20), np.float32)
+    lone[0, 0:3] = 10.0
+    both = np.concatenate([recs, lone])
+    adj = pkg.MLSMPMAdjoint([one, pkg.scene_desc(1, box)], T, T, tape="fixed")
+    for other in (1.0e7, 2.0 ** 41, 1.0e7):
+        adj.setScene(1, pkg.scene_desc(1, box, fixed_point_multiplier=other))
+        got = gradient(adj, both)
+        nan = np.isnan(want)
+        assert np.array_equal(nan, np.isnan(got))
+        assert np.array_equal(got[~nan].view(np.uint32), want[~nan].view(np.uint32)), \
+            f"beside a scene with {other}"
+    adj.close()

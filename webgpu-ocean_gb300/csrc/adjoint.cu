@@ -46,16 +46,16 @@ namespace {
 
 constexpr int kThreads = 256;
 
-// Resident CTAs per SM the particle kernels ask the register allocator for
-// (one thread per particle, unbounded: k_adj_p2g2 ~160 registers, k_adj_g2p
-// ~124; capped at 2 and 3 CTAs of 256 threads they spill 68 and 120 bytes
-// and the 1.5M-particle backward runs ~5 % faster).
-#ifndef MPM_ADJ_P2G2_MIN_BLOCKS
-#define MPM_ADJ_P2G2_MIN_BLOCKS 2
-#endif
-#ifndef MPM_ADJ_G2P_MIN_BLOCKS
-#define MPM_ADJ_G2P_MIN_BLOCKS 3
-#endif
+// Resident CTAs per SM the particle kernels ask the register allocator for.
+// The loop over a stencil's three x-slabs stays a loop where one thread walks
+// them all: unrolled 27 times the kernels outgrew the instruction cache (2.2
+// warps per issue waiting for instructions) and spilled.  64 scenes, 1.5
+// million particles (ncu, k_adj_g2p / k_adj_p2g2 / k_adj_p2g1): unrolled with 3
+// and 2 CTAs 341 / 375 / 160 us; looped 282 / 344 / 160, with dec_f<true> 268 /
+// 342 / 155, with 3 CTAs of k_adj_p2g2 too 267 / 291 / 155 (4: 288; looped
+// along y as well 270 / 310; k_adj_p2g1 at 5 CTAs 200).
+constexpr int kG2pBlocks = 3;
+constexpr int kP2g2Blocks = 3;
 
 struct Sten {
     float cf[3];     // floor(x)
@@ -118,9 +118,26 @@ __device__ __forceinline__ void store_rec(const Particles& P, int i, const Rec& 
     P.p3[i] = make_float4(r.v[0], r.v[1], r.v[2], 0.0f);
 }
 
-__device__ __forceinline__ float dec_f(int i, float fm) { return (float)i / fm; }
+// f32(i) / fm.  FAST: by RN(1 / fm), with P. Markstein's correctly rounding
+// correction of a quotient within an ulp (IBM J. Res. Dev. 34, 1990): five
+// operations instead of a division, the same bits for 2^-20 <= fm <= 2^40
+// (|i| is 0 or at least 1, so nothing underflows).  A gather decodes 81
+// velocities a particle.
+template <bool FAST>
+__device__ __forceinline__ float dec_f(int i, float fm) {
+    const float a = (float)i;
+    if (!FAST) return a / fm;
+    const float y = __frcp_rn(fm);  // the same for all cells of a scene: hoisted
+    float q = __fmul_rn(a, y);
+    q = __fmaf_rn(__fmaf_rn(-fm, q, a), y, q);
+    return __fmaf_rn(__fmaf_rn(-fm, q, a), y, q);
+}
 
-// Tape of the fixed-point solver: f32 records and the updated i32 grid.
+bool dec_is_fast(float fm) { return fm >= 0x1p-20f && fm <= 0x1p40f; }
+
+// Tape of the fixed-point solver: f32 records and the updated i32 grid.  FAST:
+// every scene's fixed-point multiplier suits dec_f<true>.
+template <bool FAST>
 struct TapeFixed {
     Particles S;
     const int4* G;
@@ -132,9 +149,9 @@ struct TapeFixed {
     // cell j (all-scene linear index): velocity (or raw momentum), mass, mass > 0
     __device__ __forceinline__ void vel(int j, float fm, float v[3]) const {
         const int4 c = __ldg(G + j);
-        v[0] = dec_f(c.x, fm); v[1] = dec_f(c.y, fm); v[2] = dec_f(c.z, fm);
+        v[0] = dec_f<FAST>(c.x, fm); v[1] = dec_f<FAST>(c.y, fm); v[2] = dec_f<FAST>(c.z, fm);
     }
-    __device__ __forceinline__ float mass(int j, float fm) const { return dec_f(__ldg(G + j).w, fm); }
+    __device__ __forceinline__ float mass(int j, float fm) const { return dec_f<FAST>(__ldg(&G[j].w), fm); }
     __device__ __forceinline__ bool updated(int j) const { return __ldg(G + j).w > 0; }
 };
 
@@ -358,7 +375,7 @@ __device__ __forceinline__ int slab_gx(int s, int q) { return L == 1 ? s : q; }
 // G = sum_n grad w_n v_n^T, H = sum_n 4 grad w_n (d_n . u_n) - 4 w_n u_n.
 // ---------------------------------------------------------------------------
 template <class Tape, int L>
-__global__ void __launch_bounds__(kThreads, MPM_ADJ_G2P_MIN_BLOCKS)
+__global__ void __launch_bounds__(kThreads, kG2pBlocks)
     k_adj_g2p(Tape tp, Particles Aout, Particles Anew, float4* __restrict__ gadj,
               const AdjScene* __restrict__ scenes, const int* __restrict__ pscene,
               const int* __restrict__ perm, int n) {
@@ -374,7 +391,7 @@ __global__ void __launch_bounds__(kThreads, MPM_ADJ_G2P_MIN_BLOCKS)
     const Rec ao = load_rec(Aout, i);
 
     float acc[15] = {};  // vg (3), G row-major (9), H (3)
-#pragma unroll
+#pragma unroll 1
     for (int s = 0; s < slab_count<L>(); ++s) {
         const Slab sx = slab(st, slab_gx<L>(s, ln.q));
 #pragma unroll
@@ -424,7 +441,7 @@ __global__ void __launch_bounds__(kThreads, MPM_ADJ_G2P_MIN_BLOCKS)
         xbar[a] += acc[3 + 3 * a] * vgbar[0] + acc[4 + 3 * a] * vgbar[1] + acc[5 + 3 * a] * vgbar[2] +
                    acc[12 + a];
 
-#pragma unroll
+#pragma unroll 1
     for (int s = 0; s < slab_count<L>(); ++s) {
         const Slab sx = slab(st, slab_gx<L>(s, ln.q));
 #pragma unroll
@@ -514,7 +531,7 @@ __global__ void __launch_bounds__(kThreads)
 // Q = sum_n w_n g_n.
 // ---------------------------------------------------------------------------
 template <class Tape, int L>
-__global__ void __launch_bounds__(kThreads, MPM_ADJ_P2G2_MIN_BLOCKS)
+__global__ void __launch_bounds__(kThreads, L == 1 ? kP2g2Blocks : 2)
     k_adj_p2g2(Tape tp, Particles Anew, float4* __restrict__ gadj,
                const AdjScene* __restrict__ scenes, const int* __restrict__ pscene,
                const int* __restrict__ perm, int n, double* __restrict__ pgrad) {
@@ -536,7 +553,7 @@ __global__ void __launch_bounds__(kThreads, MPM_ADJ_P2G2_MIN_BLOCKS)
 
     // rho (1), m grad w (3), sum w g d^T row-major (9), P1 (3), P2 (3), Q (3)
     float acc[22] = {};
-#pragma unroll
+#pragma unroll 1
     for (int s = 0; s < slab_count<L>(); ++s) {
         const Slab sx = slab(st, slab_gx<L>(s, ln.q));
 #pragma unroll
@@ -608,7 +625,7 @@ __global__ void __launch_bounds__(kThreads, MPM_ADJ_P2G2_MIN_BLOCKS)
         rhobar += pbar * k.stiffness * 5.0f * r4 / k.rest_density;
     }
     if (ln.active) {
-#pragma unroll
+#pragma unroll 1
         for (int s = 0; s < slab_count<L>(); ++s) {
             const Slab sx = slab(st, slab_gx<L>(s, ln.q));
 #pragma unroll
@@ -654,7 +671,7 @@ __global__ void __launch_bounds__(kThreads)
     Sten st;
     make_sten(p.x, st);
     float acc[15] = {};  // v adjoint (3), C adjoint C[b][a] at 3 + 3b + a (9), x adjoint (3)
-#pragma unroll
+#pragma unroll 1
     for (int s = 0; s < slab_count<L>(); ++s) {
         const Slab sx = slab(st, slab_gx<L>(s, ln.q));
 #pragma unroll
@@ -1139,10 +1156,16 @@ void adj_bricks(const SimConsts& k, int& BX, int& BY, int& BZ) {
 void launch_adjoint_substep(const Particles& S, const int4* G, const Particles& Aout,
                             const Particles& Anew, float4* gadj, const AdjScene* scenes,
                             int nscenes, const int* pscene, int n, int ncells, double* pgrad,
-                            const AdjSort& so, cudaStream_t st) {
-    adjoint_substep(TapeFixed{S, G}, Aout, Anew, gadj, scenes, nscenes, pscene, n, ncells, pgrad,
-                    so, st);
+                            const AdjSort& so, bool fast_dec, cudaStream_t st) {
+    if (fast_dec)
+        adjoint_substep(TapeFixed<true>{S, G}, Aout, Anew, gadj, scenes, nscenes, pscene, n, ncells,
+                        pgrad, so, st);
+    else
+        adjoint_substep(TapeFixed<false>{S, G}, Aout, Anew, gadj, scenes, nscenes, pscene, n, ncells,
+                        pgrad, so, st);
 }
+
+bool adj_fast_dec(const SimConsts& k) { return dec_is_fast(k.fm); }
 
 void launch_adjoint_substep64(const double* S, const double4* G, const Particles& Aout,
                               const Particles& Anew, float4* gadj, const AdjScene* scenes,

@@ -46,7 +46,10 @@ struct AdjSort {
 void launch_adjoint_substep(const Particles& S, const int4* G, const Particles& Aout,
                             const Particles& Anew, float4* gadj, const AdjScene* scenes,
                             int nscenes, const int* pscene, int n, int ncells, double* pgrad,
-                            const AdjSort& so, cudaStream_t st);
+                            const AdjSort& so, bool fast_dec, cudaStream_t st);
+
+// Whether a scene's fixed-point multiplier allows fast_dec (see dec_f).
+bool adj_fast_dec(const SimConsts& k);
 
 // The same on the FP64 tape (S: kRec64 doubles per particle; G: double4
 // cells {v or momentum, mass}).

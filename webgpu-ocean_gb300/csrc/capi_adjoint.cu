@@ -56,6 +56,7 @@ struct mpm_adjoint {
     int bg_T = -1, bg_every = 0, bg_tape = -1, bg_cur = 0;
     bool last_taped = false;         // the forward recorded its last segment's tape
     bool bg_last_taped = false;
+    bool bg_fast_dec = true;         // the kernels it was captured with (all_fast_dec)
     std::vector<int> bg_steps;
     int ncells = 0;
     std::vector<int> lbase;
@@ -264,6 +265,13 @@ int adj_lanes(long long n) {
     return n < 512LL * nsm ? 3 : 1;
 }
 
+// Every scene's fixed-point multiplier allows the kernels' fast decode.
+bool all_fast_dec(const mpm_adjoint* a) {
+    bool fast = true;
+    for (const SimConsts& k : a->b->consts) fast = fast && adj_fast_dec(k);
+    return fast;
+}
+
 // The whole backward of the last forward, enqueued on `st` (kernels,
 // memsets, device copies and event dependencies only, so it can be
 // captured): for each checkpoint segment from the last, recompute its states
@@ -280,6 +288,7 @@ int enqueue_backward(mpm_adjoint* a, const int* seed_steps, int nseeds, cudaStre
     mpm_batch* b = a->b;
     const int n = b->n, S = (int)b->consts.size();
     const bool f64 = a->tape == MPM_TAPE_FP64;
+    const bool fast_dec = all_fast_dec(a);
     const bool overlap = rs != nullptr && rs != st && a->sets == 2;
     cudaStream_t r = overlap ? rs : st;
     cudaEvent_t* ev_rec = overlap ? ev : nullptr;      // [set]: recompute into it done
@@ -356,7 +365,7 @@ int enqueue_backward(mpm_adjoint* a, const int* seed_steps, int nseeds, cudaStre
                 const Particles& Sx = t == t0 ? a->ckpt[(size_t)j] : a->seg[k][(size_t)(t - t0)];
                 launch_adjoint_substep(Sx, a->gtape[k] + (g0 + (size_t)(t - t0)) * nc, a->adj[cur],
                                        a->adj[cur ^ 1], a->gadj, a->scenes_d, S, a->pscene_d, n,
-                                       a->ncells, a->pgrad_d, a->sort, st);
+                                       a->ncells, a->pgrad_d, a->sort, fast_dec, st);
             }
             cur ^= 1;
             add_seeds(t, a->adj[cur]);
@@ -427,7 +436,8 @@ int run_backward(mpm_adjoint* a, const std::vector<int>& steps, float* grad_init
     if (b->prof.enabled) {  // per-launch profiling: no graph, one stream
         if (int rc = enqueue_backward(a, steps.data(), nseeds, st, st, nullptr, &cur)) return rc;
     } else if (a->bgraph && a->bg_T == a->T && a->bg_every == a->every && a->bg_tape == a->tape &&
-               a->bg_last_taped == a->last_taped && a->bg_steps == steps) {
+               a->bg_last_taped == a->last_taped && a->bg_fast_dec == all_fast_dec(a) &&
+               a->bg_steps == steps) {
         MPM_CUDA(cudaGraphLaunch(a->bgraph, st));
         cur = a->bg_cur;
     } else {
@@ -463,6 +473,7 @@ int run_backward(mpm_adjoint* a, const std::vector<int>& steps, float* grad_init
         a->bg_every = a->every;
         a->bg_tape = a->tape;
         a->bg_last_taped = a->last_taped;
+        a->bg_fast_dec = all_fast_dec(a);
         a->bg_steps = steps;
         a->bg_cur = cur;
         MPM_CUDA(cudaGraphLaunch(exec, st));
