@@ -174,7 +174,6 @@ struct Dev {
     uint32_t* dirty_flag[2];
     uint32_t* dirty_list[2];
     uint32_t* dirty_n;   // [2]
-    uint32_t* ticket;    // [1]
     uint32_t* bin_of;
     uint32_t* rank_of;
     uint32_t* bin_count;  // [bins + 1]
@@ -217,10 +216,15 @@ __device__ __forceinline__ uint32_t bin_base(const Scene& s) {
 
 enum { kCtrP2G2 = 0, kCtrG2P = 1, kCtrP2G1 = 2 };
 
-// Dynamic task fetch: thread 0 claims task ids from a global counter, one
-// ahead, through a two-slot shared buffer (see the loops below).
+// Dynamic task fetch: a CTA's first two tasks are its number and that plus
+// the grid's size; from then on thread 0 claims task ids from a global counter,
+// one ahead, through a two-slot shared buffer (see the loops below).  CTAs
+// without a task leave the counter alone.  With the first tasks claimed too,
+// and another counter for the last CTA to have cleared its bricks, the 608 CTAs'
+// atomics on one address took 4-7 us of every launch (ncu, 3,000 particles:
+// k_p2g2 16.5 -> 9.9 us, k_g2p_p2g1 17.0 -> 12.1 us; 200,000: k_p2g2 34 -> 27).
 __device__ __forceinline__ int claim_task(const Dev& d, int ctr) {
-    return (int)atomicAdd(d.task_next + ctr, 1u);
+    return 2 * (int)gridDim.x + (int)atomicAdd(d.task_next + ctr, 1u);
 }
 
 // Entry of claimed task t: the multi-chunk tasks (nbig of them, stored from
@@ -317,7 +321,7 @@ __device__ __forceinline__ uint32_t bin_key(const Geo& g, uint32_t base, bool re
 }
 
 // Clears the dirty bricks of grid gi (warp per brick, grid-stride over the
-// list); the last CTA to finish resets the list.
+// list); k_update, which runs next, resets the list.
 __device__ __forceinline__ void clear_dirty(const Dev& d, int gi) {
     const uint32_t nd = __ldcg(d.dirty_n + gi);
     const unsigned lane = threadIdx.x & 31u;
@@ -332,16 +336,6 @@ __device__ __forceinline__ void clear_dirty(const Dev& d, int gi) {
         vbase[lane] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         vbase[lane + 32] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (lane == 0) d.dirty_flag[gi][b] = 0u;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const uint32_t t = atomicAdd(d.ticket, 1u);
-        if (t == gridDim.x - 1) {
-            d.dirty_n[gi] = 0u;
-            *d.ticket = 0u;
-            __threadfence();
-        }
     }
 }
 
@@ -512,8 +506,8 @@ __global__ void __launch_bounds__(TH, 1024 / TH)
     for (int i = threadIdx.x; i < NB * 3 * kNA; i += TH) (&s_q[0][0][0])[i] = 0;
     if (threadIdx.x < 33) s_lt.cnt[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
-        s_task[0] = claim_task(d, kCtrP2G2);
-        s_task[1] = claim_task(d, kCtrP2G2);
+        s_task[0] = (int)blockIdx.x;
+        s_task[1] = (int)(blockIdx.x + gridDim.x);
     }
 
     // offsets of this thread's arena slots for geometry class off_class
@@ -704,6 +698,8 @@ __global__ void __launch_bounds__(TH, 1024 / TH)
 // ---------------------------------------------------------------------------
 template <bool BATCH>
 __global__ void __launch_bounds__(256) k_update(Scene one, Dev d, int cur) {
+    // the other grid's dirty bricks were cleared by k_p2g2
+    if (blockIdx.x == 0 && threadIdx.x == 0) d.dirty_n[cur ^ 1] = 0u;
     const uint32_t nd = __ldcg(d.dirty_n + cur);
     const unsigned lane = threadIdx.x & 31u;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -782,8 +778,8 @@ __global__ void __launch_bounds__(TH, 1024 / TH)
     for (int i = threadIdx.x; i < NB * 4 * kNB; i += TH) (&s_a[0][0][0])[i] = 0;
     if (threadIdx.x < NB * kTouch) (&s_touch[0][0])[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
-        s_task[0] = claim_task(d, ctr);
-        s_task[1] = claim_task(d, ctr);
+        s_task[0] = (int)blockIdx.x;
+        s_task[1] = (int)(blockIdx.x + gridDim.x);
     }
 
     // offsets of this thread's arena slots for geometry class off_class /
@@ -1522,7 +1518,6 @@ int sorted_create(SortedEngine** out, int max_particles) {
     if (r == cudaSuccess) r = cudaMalloc(&e->d.rank_of, 4 * np);
     if (r == cudaSuccess) r = cudaMalloc(&e->d.order, 4 * np);
     if (r == cudaSuccess) r = cudaMalloc(&e->d.dirty_n, 4 * 2);
-    if (r == cudaSuccess) r = cudaMalloc(&e->d.ticket, 4);
     if (r == cudaSuccess) r = cudaMalloc(&e->d.ntasks, 4 * 2);
     if (r == cudaSuccess) r = cudaMalloc(&e->d.task_next, 4 * 3);
     if (r == cudaSuccess) {
@@ -1554,7 +1549,6 @@ void sorted_destroy(SortedEngine* e) {
     cudaFree(e->d.rank_of);
     cudaFree(e->d.order);
     cudaFree(e->d.dirty_n);
-    cudaFree(e->d.ticket);
     cudaFree(e->d.ntasks);
     cudaFree(e->d.task_next);
     delete e;
@@ -1856,7 +1850,6 @@ int prime(SortedEngine* e, ParticleStore* ps, float4* posvel, unsigned long long
         SE_CUDA(cudaMemsetAsync(e->d.dirty_flag[b], 0, 4 * (size_t)e->nbricks, st));
     }
     SE_CUDA(cudaMemsetAsync(e->d.dirty_n, 0, 8, st));
-    SE_CUDA(cudaMemsetAsync(e->d.ticket, 0, 4, st));
     SE_CUDA(cudaMemsetAsync(e->d.task_next, 0, 4 * 3, st));
     // k_chunk_sums reads the whole last chunk: the counts past nbins stay zero
     SE_CUDA(cudaMemsetAsync(e->d.bin_count, 0, 4 * ((size_t)nbins + kScanThreads), st));
