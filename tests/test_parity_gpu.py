@@ -537,3 +537,23 @@ def test_pipelined_posvel_readback(cuda, pkg):
     sim.waitPosvel(stream)
     stream.synchronize()
     sim.close()
+
+
+@pytest.mark.parametrize("box", [(24, 12, 56), (16, 16, 64), (32, 32, 32), (128, 128, 124), (128, 128, 128)])
+def test_scan_chunk_edges(cuda, pkg, oracle_mod, box):
+    """Bin counts on either side of a scan chunk (254, 258, 514 bins of 256 a
+    chunk) and of the chunk sums' use (31,746 and 32,770 bins: 125 and 129
+    chunks), particles over the whole box, some bins of several tasks."""
+    rng = np.random.default_rng(box[2])
+    recs = np.zeros((5000, 20), np.float32)
+    recs[:, 0:3] = 2.0 + rng.random((5000, 3)) * (np.array(box) - 4.5)
+    recs[:1500, 0:3] = np.array(box) - 6.0 + rng.random((1500, 3))
+    recs[:, 4:7] = rng.normal(0.0, 0.5, (5000, 3))
+    sim = make_sim(pkg, "sorted", max_particles=5000, max_grid=box)
+    sim.upload(recs, [float(b) for b in box])
+    ref = oracle_mod.OracleSim(sim.downloadParticles(), [float(b) for b in box])
+    for _ in range(2):
+        sim.execute()
+        ref.execute(2, NTHREADS)
+    assert_state_equal(sim, ref, f"box {box}")
+    sim.close()

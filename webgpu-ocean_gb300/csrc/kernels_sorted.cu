@@ -96,10 +96,15 @@ constexpr int kPairSlot = 1 << 30;
 // 256, 512, all).
 constexpr int kPairMaxDefault = 512;
 constexpr int kPairDefaultRequest = INT_MAX;  // sorted_set_pair_max: restore the default
-constexpr int kScanThreads = 1024;
+// Bins per CTA of the scan.  Few, because a bin's share of the scan and its
+// tasks are ~500 instructions: with 1024 bins a CTA a scene of 3,000 bins ran
+// them on four SMs (ncu: k_scan at 200,000 particles 9.9 -> 4.7 us, at 3,000
+// 5.9 -> 3.6 us, at a million 8.6 -> 4.4 us and 3.2 us for the chunk sums).
+constexpr int kScanThreads = 256;
 // With more bin chunks (of kScanThreads bins) than this, k_chunk_sums sums
-// each chunk once before k_scan.
-constexpr int kChunkedScanMin = 64;
+// each chunk once before k_scan (a million particles, 133 chunks: frame 376 us
+// with the chunk sums, 393 us with every CTA adding up the bins before its own).
+constexpr int kChunkedScanMin = 128;
 // A bin holding more than `task_cap` particles is split into tasks of at
 // most task_cap particles (same brick, separate arena flushes), so that small
 // scenes, whose bricks are few and full, still spread over every SM.
@@ -1077,8 +1082,10 @@ __global__ void __launch_bounds__(kTask) k_bin(Particles P, Scene one, Dev d, in
 // itself (a few KB to a few hundred KB from L2), so no CTA waits on another.
 // The counts are zeroed by k_scatter, which runs next.
 
+constexpr int kScanWarps = kScanThreads / 32;
+
 // Block-wide exclusive scan of N values per thread, in place; tot gets the
-// block's totals.  s: 32 * N words of shared scratch.
+// block's totals.  s: kScanWarps * N words of shared scratch.
 template <int N>
 __device__ __forceinline__ void block_scan(uint32_t (&v)[N], uint32_t (&tot)[N], uint32_t* s) {
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -1095,26 +1102,38 @@ __device__ __forceinline__ void block_scan(uint32_t (&v)[N], uint32_t (&tot)[N],
     }
     if (lane == 31) {
 #pragma unroll
-        for (int k = 0; k < N; ++k) s[k * 32 + warp] = inc[k];
-    }
-    __syncthreads();
-    if (warp == 0) {
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-            uint32_t w = s[k * 32 + lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-                if ((int)lane >= o) w += y;
-            }
-            s[k * 32 + lane] = w;
-        }
+        for (int k = 0; k < N; ++k) s[k * kScanWarps + warp] = inc[k];
     }
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < N; ++k) {
-        tot[k] = s[k * 32 + 31];
-        v[k] = inc[k] - v[k] + (warp ? s[k * 32 + warp - 1] : 0u);
+        uint32_t before = 0u, all = 0u;
+#pragma unroll
+        for (int w = 0; w < kScanWarps; ++w) {
+            const uint32_t x = s[k * kScanWarps + w];
+            if (w < (int)warp) before += x;
+            all += x;
+        }
+        tot[k] = all;
+        v[k] = before + inc[k] - v[k];
+    }
+}
+
+// Block-wide sums, for every thread.
+template <int N>
+__device__ __forceinline__ void block_sum(uint32_t (&v)[N], uint32_t* s) {
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const uint32_t x = __reduce_add_sync(0xffffffffu, v[k]);
+        if (lane == 0) s[k * kScanWarps + warp] = x;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        v[k] = 0u;
+#pragma unroll
+        for (int w = 0; w < kScanWarps; ++w) v[k] += s[k * kScanWarps + w];
     }
 }
 
@@ -1176,6 +1195,7 @@ __device__ __forceinline__ void sum_bins(const Dev& d, int b0, int b1, uint32_t 
         }
 #pragma unroll
         for (int u = 0; u < kU; ++u) {  // two z pairs each
+            if (i0 + u * kScanThreads >= n4) break;  // uniform
             uint32_t bg, sm;
             pair_tasks(d, q[u].x, q[u].y, bg, sm);
             pre[1] += bg;
@@ -1186,18 +1206,14 @@ __device__ __forceinline__ void sum_bins(const Dev& d, int b0, int b1, uint32_t 
             pre[0] += q[u].x + q[u].y + q[u].z + q[u].w;
         }
     }
-    uint32_t tot[3];
-    block_scan<3>(pre, tot, s_scan);
-    pre[0] = tot[0];
-    pre[1] = tot[1];
-    pre[2] = tot[2];
+    block_sum<3>(pre, s_scan);
 }
 
 // Per-chunk sums for k_scan when there are many chunks (otherwise each
 // k_scan CTA reduces all earlier bins itself, which costs a quadratic
 // number of reads).  The bin counts beyond nbins are zero.
 __global__ void __launch_bounds__(kScanThreads) k_chunk_sums(Dev d) {
-    __shared__ uint32_t s_scan[3 * 32];
+    __shared__ uint32_t s_scan[3 * kScanWarps];
     uint32_t pre[3];
     sum_bins(d, blockIdx.x * kScanThreads, (blockIdx.x + 1) * kScanThreads, pre, s_scan);
     if (threadIdx.x < 3) d.chunk_sum[3 * blockIdx.x + threadIdx.x] = pre[threadIdx.x];
@@ -1205,7 +1221,7 @@ __global__ void __launch_bounds__(kScanThreads) k_chunk_sums(Dev d) {
 
 // chunked: k_chunk_sums ran before (chunk_sum holds every chunk's sums).
 __global__ void __launch_bounds__(kScanThreads) k_scan(Dev d, Geo one_g, int nbins, int chunked) {
-    __shared__ uint32_t s_scan[3 * 32];
+    __shared__ uint32_t s_scan[3 * kScanWarps];
     const int base = blockIdx.x * kScanThreads;
     // counts of all bins before this CTA's range (particles, big and small tasks)
     uint32_t pre[3] = {0u, 0u, 0u};
@@ -1213,11 +1229,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Dev d, Geo one_g, int nbi
         for (int c = threadIdx.x; c < (int)blockIdx.x; c += kScanThreads)
 #pragma unroll
             for (int k = 0; k < 3; ++k) pre[k] += __ldcg(d.chunk_sum + 3 * c + k);
-        uint32_t tot[3];
-        block_scan<3>(pre, tot, s_scan);
-        pre[0] = tot[0];
-        pre[1] = tot[1];
-        pre[2] = tot[2];
+        block_sum<3>(pre, s_scan);
     } else {
         sum_bins(d, 0, base, pre, s_scan);
     }
