@@ -557,3 +557,24 @@ def test_scan_chunk_edges(cuda, pkg, oracle_mod, box):
         ref.execute(2, NTHREADS)
     assert_state_equal(sim, ref, f"box {box}")
     sim.close()
+
+
+def test_constants_that_change_between_calls(cuda, pkg, oracle_mod):
+    """Calls that keep the constants replay a graph, calls that change them
+    launch their kernels: walls moving every frame, resting, moving while
+    graphs are switched off, and back."""
+    box = [30.0, 24.0, 40.0]
+    sim = make_sim(pkg, "sorted")
+    sim.reset(6000, box)
+    ref = oracle_mod.OracleSim(sim.downloadParticles(), box)
+    real = list(box)
+    for frame in range(24):
+        sim.setGraph(not 10 <= frame < 16)
+        if 4 <= frame < 8 or frame in (12, 18):
+            real[2] -= 0.7
+        sim.changeBoxSize(real)
+        ref.change_box_size(real)
+        sim.execute()
+        ref.execute(2, NTHREADS)
+    assert_state_equal(sim, ref, "after 24 frames")
+    sim.close()
