@@ -248,6 +248,7 @@ __global__ void __launch_bounds__(kBinBlock)
 
 // First entries of the tiles and the work items, one block.
 __global__ void __launch_bounds__(1024) k_tile_scan(Bins bins, uint32_t per) {
+    constexpr uint32_t kOwn = 4;  // items of a tile that its thread writes
     __shared__ uint32_t s_w[2][32];
     const int tiles = bins.tx * bins.ty;
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -287,8 +288,19 @@ __global__ void __launch_bounds__(1024) k_tile_scan(Bins bins, uint32_t per) {
         if (t < tiles) {
             bins.cursor[t] = before[0];
             if (c) bins.count[t] = 0u;
-            for (uint32_t k = 0; k < x[1]; ++k)
-                bins.item[before[1] + k] = Item{t, (int)(before[0] + k * per), (int)min(c - k * per, per)};
+#pragma unroll
+            for (uint32_t k = 0; k < kOwn; ++k)
+                if (k < x[1])
+                    bins.item[before[1] + k] = Item{t, (int)(before[0] + k * per), (int)min(c - k * per, per)};
+        }
+        // tiles with more have dozens: their other items by the whole warp
+        for (unsigned left = __ballot_sync(0xffffffffu, x[1] > kOwn); left; left &= left - 1u) {
+            const int src = __ffs((int)left) - 1;
+            const uint32_t count = __shfl_sync(0xffffffffu, c, src);
+            const uint32_t first = __shfl_sync(0xffffffffu, before[0], src);
+            const uint32_t at = __shfl_sync(0xffffffffu, before[1], src);
+            for (uint32_t k = kOwn + lane; k * per < count; k += 32)
+                bins.item[at + k] = Item{t - (int)lane + src, (int)(first + k * per), (int)min(count - k * per, per)};
         }
     }
     if (threadIdx.x == 0) {
@@ -509,10 +521,12 @@ __global__ void __launch_bounds__(kTileBlock)
                 const float r2 = add(mul(nx, nx), ny2);
                 if (r2 > 1.0f) continue;
                 const float nz = __fsqrt_rn(sub(1.0f, r2));
-                if (THICK) {  // below 2^28: 32 bits and a carry
+                if (THICK) {
+                    // below 2^28, in two parts whose sums over an item's
+                    // billboards fit 32 bits: additions that return nothing
                     const uint32_t v = __float2uint_rn(mul(mul(0.05f, nz), 4294967296.0f));
-                    const uint32_t old = atomicAdd(s_lo + p, v);
-                    if (old + v < old) atomicAdd(s_hi + p, 1u);
+                    atomicAdd(s_lo + p, v & 0x3fffu);
+                    atomicAdd(s_hi + p, v >> 14);
                     if (behind) continue;
                 }
                 const float z = add(t.view_z, mul(nz, radius));
@@ -543,7 +557,7 @@ __global__ void __launch_bounds__(kTileBlock)
             if (THICK) {
                 const uint32_t lo = s_lo[p], hi = s_hi[p];
                 if (lo | hi) {
-                    atomicAdd(tacc + q, (unsigned long long)hi << 32 | lo);
+                    atomicAdd(tacc + q, ((unsigned long long)hi << 14) + lo);
                     s_lo[p] = s_hi[p] = 0u;
                 }
             }
