@@ -9,9 +9,9 @@
 //                     thicknessMap.wgsl:27-62]
 //   k_resolve         depth map (view z of the nearest fragment) and the
 //                     thickness map (r16float)
-//   k_bilateral x 8   separable bilateral filter of the depth map, 4 x (X, Y)
-//                     [bilateral.wgsl:18-75]
-//   k_gaussian x 2    separable gaussian of the thickness map, (X, Y)
+//   k_filter x 8      separable bilateral filter of the depth map, 4 x (X, Y)
+//                     [bilateral.wgsl:18-75], and with its first two passes the
+//                     separable gaussian of the thickness map, (X, Y)
 //                     [gaussian.wgsl:14-42]
 //   k_shade           normals, lighting, fresnel, transmittance, cube-map
 //                     reflection [fluid.wgsl:37-98]
@@ -672,17 +672,25 @@ __device__ __forceinline__ DepthWeight depth_weight(const Consts& c) {
 // arithmetic, and the taps' weights have no branch, so that several overlap.
 // Per pass (ncu) at 896x504 15.5 -> 12.0 us, at 1344x756 20.9 -> 16.8 us;
 // shared memory alone 13.3 and 18.3.
-constexpr int kBilThreads = 256;
+constexpr int kFilterThreads = 256;
 
 template <bool X>
-__global__ void __launch_bounds__(kBilThreads)
-    k_bilateral(const float* __restrict__ src, float* __restrict__ dst, Consts c,
-                const float* __restrict__ wtab) {
-    constexpr int kW = X ? 256 : 32, kH = kBilThreads / kW;  // pixels of a block
-    __shared__ float s_d[X ? kW + 2 * kMaxFs : kW * (kH + 2 * kMaxFs)];
-    __shared__ int s_fs;
+struct Bilateral {
+    static constexpr int kW = X ? 256 : 32, kH = kFilterThreads / kW;  // pixels of a block
+    float d[X ? kW + 2 * kMaxFs : kW * (kH + 2 * kMaxFs)];             // shared memory
+    int fs;
+};
+
+template <bool X>
+__device__ __forceinline__ void bilateral_block(Bilateral<X>& sm, int block,
+                                                const float* __restrict__ src,
+                                                float* __restrict__ dst, const Consts& c,
+                                                const float* __restrict__ wtab) {
+    constexpr int kW = Bilateral<X>::kW, kH = Bilateral<X>::kH;
+    float* s_d = sm.d;
+    int& s_fs = sm.fs;
     const int columns = (c.W + kW - 1) / kW;
-    const int bx = (int)blockIdx.x % columns * kW, by = (int)blockIdx.x / columns * kH;
+    const int bx = block % columns * kW, by = block / columns * kH;
     const int lx = (int)threadIdx.x % kW, ly = (int)threadIdx.x / kW;
     const int px = bx + lx, py = by + ly;
     const bool in = px < c.W && py < c.H;
@@ -701,10 +709,10 @@ __global__ void __launch_bounds__(kBilThreads)
     const int halo = s_fs;  // <= max_filter_size = kMaxFs
     if (halo < 0) return;   // uniform
     if (X) {
-        for (int k = threadIdx.x; k < kW + 2 * halo; k += kBilThreads)
+        for (int k = threadIdx.x; k < kW + 2 * halo; k += kFilterThreads)
             s_d[k] = fabsf(src[(size_t)by * c.W + clampi(bx - halo + k, 0, c.W - 1)]);
     } else {
-        for (int k = threadIdx.x; k < kW * (kH + 2 * halo); k += kBilThreads)
+        for (int k = threadIdx.x; k < kW * (kH + 2 * halo); k += kFilterThreads)
             s_d[k] = fabsf(src[(size_t)clampi(by - halo + k / kW, 0, c.H - 1) * c.W +
                                min(bx + k % kW, c.W - 1)]);
     }
@@ -737,20 +745,26 @@ __global__ void __launch_bounds__(kBilThreads)
 // shared memory, so that a tap costs a product, a sum and half a load.  The
 // weights' sum is the same for every pixel and was made with the table.  Per
 // pass (ncu) at 896x504 15.8 -> 9.3 us, at 1344x756 26.7 -> 12.5 us.
-constexpr int kGaussThreads = 256;
+template <bool X>
+struct Gaussian {
+    // along x: 4 rows of 256 pixels; along y: 32 rows of 32 pixels
+    static constexpr int kW = X ? 256 : 32, kH = X ? 4 : 32;
+    static constexpr int kSW = X ? kW + 2 * kGaussFs + 4 : kW, kSH = X ? kH : kH + 2 * kGaussFs;
+    alignas(16) float t[kSH * kSW];  // shared memory
+    alignas(16) float g[64];
+};
 
 template <bool X>
-__global__ void __launch_bounds__(kGaussThreads)
-    k_gaussian(const float* __restrict__ src, float* __restrict__ dst, Consts c,
-               const float* __restrict__ gtab) {
+__device__ __forceinline__ void gaussian_block(Gaussian<X>& sm, int block,
+                                               const float* __restrict__ src,
+                                               float* __restrict__ dst, const Consts& c,
+                                               const float* __restrict__ gtab) {
     constexpr int kTaps = 2 * kGaussFs + 1, kOut = 4;
-    // along x: 4 rows of 256 pixels; along y: 32 rows of 32 pixels
-    constexpr int kW = X ? 256 : 32, kH = X ? 4 : 32;
-    constexpr int kSW = X ? kW + 2 * kGaussFs + 4 : kW, kSH = X ? kH : kH + 2 * kGaussFs;
-    __shared__ __align__(16) float s_t[kSH * kSW];
-    __shared__ __align__(16) float s_g[64];
+    constexpr int kW = Gaussian<X>::kW, kH = Gaussian<X>::kH, kSW = Gaussian<X>::kSW,
+                  kSH = Gaussian<X>::kSH;
+    float *s_t = sm.t, *s_g = sm.g;
     const int columns = (c.W + kW - 1) / kW;
-    const int bx = (int)blockIdx.x % columns * kW, by = (int)blockIdx.x / columns * kH;
+    const int bx = block % columns * kW, by = block / columns * kH;
     // this thread's first pixel, from the block's corner
     const int lx = X ? kOut * ((int)threadIdx.x & 63) : (int)threadIdx.x & 31;
     const int ly = X ? (int)threadIdx.x >> 6 : kOut * ((int)threadIdx.x >> 5);
@@ -758,7 +772,7 @@ __global__ void __launch_bounds__(kGaussThreads)
         const int o = (int)threadIdx.x - kGaussFs;
         s_g[threadIdx.x] = threadIdx.x < kTaps ? gtab[o < 0 ? -o : o] : 0.0f;
     }
-    for (int k = threadIdx.x; k < kSH * kSW; k += kGaussThreads) {
+    for (int k = threadIdx.x; k < kSH * kSW; k += kFilterThreads) {
         const int x = bx + k % kSW - (X ? kGaussFs : 0), y = by + k / kSW - (X ? 0 : kGaussFs);
         s_t[k] = src[(size_t)clampi(y, 0, c.H - 1) * c.W + clampi(x, 0, c.W - 1)];
     }
@@ -807,6 +821,30 @@ __global__ void __launch_bounds__(kGaussThreads)
         if (px < c.W && py < c.H)
             dst[(size_t)py * c.W + px] = centre[i] == 0.0f ? 0.0f : half_round(dvd(sum[i], wsum));
     }
+}
+
+// A bilateral pass over `depth` and, in the blocks after its own (if there are
+// any), the gaussian pass along the same axis over `thick`.  The two images'
+// chains do not depend on each other, and either's launches leave most of the
+// GPU's issue slots unused: the gaussian's 16.5 us (ncu, 896x504; 22.8 at
+// 1344x756) run in the first two bilateral launches' shadow.
+struct FilterPass {
+    const float* src;
+    float* dst;
+};
+
+template <bool X>
+__global__ void __launch_bounds__(kFilterThreads)
+    k_filter(FilterPass depth, FilterPass thick, int depth_blocks, Consts c,
+             const float* __restrict__ wtab, const float* __restrict__ gtab) {
+    __shared__ __align__(16) union {
+        Bilateral<X> bilateral;
+        Gaussian<X> gaussian;
+    } sm;
+    if ((int)blockIdx.x < depth_blocks)
+        bilateral_block<X>(sm.bilateral, (int)blockIdx.x, depth.src, depth.dst, c, wtab);
+    else
+        gaussian_block<X>(sm.gaussian, (int)blockIdx.x - depth_blocks, thick.src, thick.dst, c, gtab);
 }
 
 // fluid.wgsl:19-27: view-space position from a texture coordinate and depth.
@@ -1223,13 +1261,16 @@ int mpm_renderer_execute(mpm_renderer* r, const void* posvel, int n,
     k_resolve<<<pb, 256, 0, st>>>(pv, u, c, r->dkey, r->tacc, r->depth[0], r->thick[0]);
     // blocks of w x h pixels, row by row (one grid dimension: images of one column have 2^28 rows)
     const auto grid = [&](int w, int h) { return (unsigned)((c.W + w - 1) / w) * (unsigned)((c.H + h - 1) / h); };
-    const unsigned bx = grid(256, 1), by = grid(32, kBilThreads / 32);
-    for (int it = 0; it < 4; ++it) {  // fluidRender.ts:455-466
-        k_bilateral<true><<<bx, kBilThreads, 0, st>>>(r->depth[0], r->depth[1], c, r->wtab);
-        k_bilateral<false><<<by, kBilThreads, 0, st>>>(r->depth[1], r->depth[0], c, r->wtab);
+    const unsigned bx = grid(Bilateral<true>::kW, Bilateral<true>::kH);
+    const unsigned by = grid(Bilateral<false>::kW, Bilateral<false>::kH);
+    for (int it = 0; it < 4; ++it) {  // fluidRender.ts:455-466, and once :474-486
+        const unsigned gx = it ? 0u : grid(Gaussian<true>::kW, Gaussian<true>::kH);
+        const unsigned gy = it ? 0u : grid(Gaussian<false>::kW, Gaussian<false>::kH);
+        k_filter<true><<<bx + gx, kFilterThreads, 0, st>>>({r->depth[0], r->depth[1]}, {r->thick[0], r->thick[1]},
+                                                          (int)bx, c, r->wtab, r->gtab);
+        k_filter<false><<<by + gy, kFilterThreads, 0, st>>>({r->depth[1], r->depth[0]}, {r->thick[1], r->thick[0]},
+                                                           (int)by, c, r->wtab, r->gtab);
     }
-    k_gaussian<true><<<grid(256, 4), kGaussThreads, 0, st>>>(r->thick[0], r->thick[1], c, r->gtab);  // :474-486
-    k_gaussian<false><<<grid(32, 32), kGaussThreads, 0, st>>>(r->thick[1], r->thick[0], c, r->gtab);
     k_shade<<<pb, 256, 0, st>>>(r->depth[0], r->thick[0], r->env, r->env_size, u, c, r->color,
                                 r->color8);
     const cudaError_t e = cudaGetLastError();
