@@ -146,13 +146,13 @@ constexpr int kMaxChunks = 256;  // 62^3 cells: 233
 // of a settled pool share a few dozen chunks).  Particles outside the grid
 // keep zero densities (density.wgsl:58-59) and so a zero force (force.wgsl) and
 // their place; the others' results come from the force kernels.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(1024)
     k_sph_bin(SphOut out, int n, Env e, int* __restrict__ cell_of, unsigned* __restrict__ count,
               unsigned* __restrict__ chunk, unsigned* __restrict__ rank) {
     __shared__ unsigned s_chunk[kMaxChunks];
-    for (int k = threadIdx.x; k < kMaxChunks; k += 256) s_chunk[k] = 0u;
+    for (int k = threadIdx.x; k < kMaxChunks; k += blockDim.x) s_chunk[k] = 0u;
     __syncthreads();
-    const int i = blockIdx.x * 256 + threadIdx.x;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
         float4 p = out.P[i];
         int xi, yi, zi;
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(256)
         }
     }
     __syncthreads();
-    for (int k = threadIdx.x; k < kMaxChunks; k += 256)
+    for (int k = threadIdx.x; k < kMaxChunks; k += blockDim.x)
         if (s_chunk[k]) atomicAdd(chunk + k, s_chunk[k]);
 }
 
@@ -395,7 +395,7 @@ __device__ __forceinline__ void neighbour_row(const Env& e, const unsigned* __re
 // bits.  Per two-substep frame of settled pools, with one warp (10,000
 // particles) or one thread per particle testing and computing as it goes, and
 // now (the sort's launches included): 10,000 particles 169 -> 55 us, 40,000
-// 308 -> 96 us, 400,000 1830 -> 730 us.
+// 308 -> 97 us, 400,000 1830 -> 669 us.
 // ---------------------------------------------------------------------------
 
 // Neighbours listed per particle (a settled pool has 25-60, its bottom up to
@@ -540,20 +540,24 @@ __global__ void __launch_bounds__(kGroupBlock)
 // ballot and the terms no trip through shared memory (290 instead of 614
 // warp instructions per particle), at a few warps per scheduler.  The list of a
 // round is the thread's own column in shared memory; 32 entries, because more
-// would take the L1 cache that the candidates' positions live in (64 entries
-// and one candidate loaded at a time: 264 instead of 177 us at 400,000
-// particles).  The lanes of a warp (neighbouring
-// sorted slots) take their terms together, when some lane's list is full and at
-// the end: a lane that took its terms alone would hold up the other 31.
+// would cost resident warps (64 entries and one candidate loaded at a time from
+// global memory: 264 us at 400,000 particles).  The lanes of a warp
+// (neighbouring sorted slots) take their terms together, when some lane's list
+// is full and at the end: a lane that took its terms alone would hold up the
+// other 31.  They share most of a row's candidates too, so the warp fetches the
+// row's run once (four candidates a thread from global memory: 181 us; from the
+// run: 171; and four neighbours' positions loaded ahead of their terms: 164).
 constexpr int kThreadBlock = 128;
 constexpr int kThreadList = 32;
-constexpr int kThreadStep = 4;  // candidates loaded at a time
+constexpr int kThreadStep = 4;  // candidates between two looks at the lists
+constexpr int kRowCache = 96;  // candidates of a row that a warp keeps
 
 __global__ void __launch_bounds__(kThreadBlock)
     k_sph_density_thread(const float4* __restrict__ SP, const float4* __restrict__ SV,
                          float4* __restrict__ D, float2* __restrict__ DR, NeighbourLists nl,
                          const unsigned* __restrict__ start, Env e) {
     __shared__ unsigned s_j[kThreadList][kThreadBlock];
+    __shared__ float4 s_row[kThreadBlock / 32][kRowCache];
     const int nbin = (int)start[e.total];
     const int s = blockIdx.x * kThreadBlock + threadIdx.x;
     if ((s & ~31) >= nbin) return;  // uniform per warp
@@ -565,30 +569,53 @@ __global__ void __launch_bounds__(kThreadBlock)
     float dens = 0.0f, near = 0.0f;
     int m = 0, taken = 0;
     auto take = [&]() {
-#pragma unroll 2
-        for (int k = 0; k < m; ++k) {
-            const unsigned j = s_j[k][threadIdx.x];
-            nl.put(s, taken + k, j);
-            const float r = __fsqrt_rn(dist2(pi, SP[j]));
-            dens = add(dens, mul(e.mass, density_kernel(e, r)));
-            near = add(near, mul(e.mass, near_density_kernel(e, r)));
+        for (int k0 = 0; k0 < m; k0 += 4) {
+            unsigned j[4];
+            float4 p[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) j[q] = k0 + q < m ? s_j[k0 + q][threadIdx.x] : 0u;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) p[q] = SP[j[q]];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (k0 + q >= m) break;
+                nl.put(s, taken + k0 + q, j[q]);
+                const float r = __fsqrt_rn(dist2(pi, p[q]));
+                dens = add(dens, mul(e.mass, density_kernel(e, r)));
+                near = add(near, mul(e.mass, near_density_kernel(e, r)));
+            }
         }
         taken += m;
         m = 0;
         __syncwarp();
     };
+    float4* row_p = s_row[threadIdx.x >> 5];
+    const unsigned lane = threadIdx.x & 31u;
     for (int row = 0; row < 9; ++row) {
         unsigned b = 0u, en = 0u;
         if (in) neighbour_row(e, start, vx, vy, vz, row, b, en);
-        while (__any_sync(0xffffffffu, b < en)) {
-            if (__any_sync(0xffffffffu, m > kThreadList - kThreadStep)) take();
-            float4 p[kThreadStep];
+        const unsigned lo = __reduce_min_sync(0xffffffffu, b < en ? b : 0xffffffffu);
+        const unsigned hi = __reduce_max_sync(0xffffffffu, en);
+        if (lo >= hi) continue;  // uniform
+        auto walk = [&](auto&& at) {
+            while (__any_sync(0xffffffffu, b < en)) {
+                if (__any_sync(0xffffffffu, m > kThreadList - kThreadStep)) take();
+                float4 p[kThreadStep];
 #pragma unroll
-            for (int q = 0; q < kThreadStep; ++q) p[q] = SP[min(b + q, (unsigned)nbin - 1u)];
+                for (int q = 0; q < kThreadStep; ++q) p[q] = at(b + q);
 #pragma unroll
-            for (int q = 0; q < kThreadStep; ++q)
-                if (b + q < en && dist2(pi, p[q]) < e.kr2) s_j[m++][threadIdx.x] = b + q;
-            b += kThreadStep;
+                for (int q = 0; q < kThreadStep; ++q)
+                    if (b + q < en && dist2(pi, p[q]) < e.kr2) s_j[m++][threadIdx.x] = b + q;
+                b += kThreadStep;
+            }
+        };
+        if (hi - lo <= kRowCache) {
+            __syncwarp();
+            for (unsigned k = lane; k < hi - lo; k += 32) row_p[k] = SP[lo + k];
+            __syncwarp();
+            walk([&](unsigned j) { return row_p[min(j - lo, (unsigned)kRowCache - 1u)]; });
+        } else {
+            walk([&](unsigned j) { return SP[min(j, (unsigned)nbin - 1u)]; });
         }
     }
     take();
@@ -761,9 +788,10 @@ struct SplitMix64 {
 
 // Which density and force kernels run at n particles.  Frames in us, settled
 // pools (16 lanes / 8 lanes / 8 lanes for the densities and a thread for the
-// forces / a thread for both): 8,000 particles 51 / 54 / 66 / 101, 12,000 60 /
-// 60 / 69 / 109, 24,000 87 / 83 / 81 / 119, 100,000 268 / 222 / 182 / 190,
-// 130,000 330 / 281 / 229 / 225, 400,000 - / 1097 / 836 / 758: the fewer the
+// forces / a thread for both, the last before it shared rows): 8,000 particles
+// 51 / 54 / 66 / 101, 12,000 60 / 60 / 69 / 109, 24,000 87 / 83 / 81 / 119,
+// 100,000 268 / 222 / 182 / 190, 130,000 330 / 281 / 229 / 225, 400,000 - /
+// 1097 / 836 / 758 (696 with them): the fewer the
 // particles, the more lanes it takes to hide a particle's chain of loads, and
 // the more of them the fewer instructions decide.
 constexpr int kSph16Max = 12000;
@@ -1034,7 +1062,10 @@ void enqueue_substeps(mpm_sph* s, int substeps, cudaStream_t st) {
     const int pb = (n + 255) / 256;
     const int chunks = (e.total + kScan - 1) / kScan;
     for (int k = 0; k < substeps; ++k) {
-        k_sph_bin<<<pb, 256, 0, st>>>(out, n, e, s->cell_of, s->count, s->chunk, s->rank);
+        // big blocks where there are enough of them: fewer blocks add to the few
+        // chunk counts (ncu, 400,000 particles: 14.1 -> 11.3 us)
+        const int bin_block = n >= 200000 ? 1024 : 256;
+        k_sph_bin<<<(n + bin_block - 1) / bin_block, bin_block, 0, st>>>(out, n, e, s->cell_of, s->count, s->chunk, s->rank);
         k_sph_scan<<<chunks, kScan, 0, st>>>(s->count, s->chunk, e.total, s->start);
         k_sph_scatter<<<pb, 256, 0, st>>>(s->cell_of, s->rank, s->start, n, s->chunk, s->arrival);
         // sorted slots: start[total] of them (read on the device); launched
