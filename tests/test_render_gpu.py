@@ -285,3 +285,59 @@ def test_filters(cuda, pkg, oracle_mod, W, H, radius, dist):
     for k in ("depth", "thickness", "color", "color8"):
         same_bits(r.download(k), want[k], k)
     r.close()
+
+
+def test_images_in_a_row(cuda, pkg):
+    """An image's launches overlap one another, not what stands before and
+    after them in the stream: images behind writes of their particles, on a
+    side stream and replayed from a captured graph, are those drawn one at a
+    time."""
+    import torch
+    W, H = 150, 110
+    u = pkg.camera_uniforms(W, H, 40.0, [10.0, 4.0, 12.0], FOV, 1.2)
+    pools = [torch.from_numpy(pool(5000, (20.0, 8.0, 24.0), s)).cuda() for s in range(4)]
+    modes = [True, False, False, True]
+    r = pkg.FluidRenderer(W, H, RADIUS, FOV)
+    want = []
+    for p, spheres in zip(pools, modes):
+        torch.cuda.synchronize()
+        r.execute(p, len(p), u, sphereRenderFl=spheres)
+        torch.cuda.synchronize()
+        want.append([r.download(k) for k in ("color", "depth")])
+    r.close()
+
+    pv = torch.zeros_like(pools[0])
+    rs = [pkg.FluidRenderer(W, H, RADIUS, FOV) for _ in pools]
+    last = pkg.FluidRenderer(W, H, RADIUS, FOV)  # draws all of them, one over the other
+    stream = torch.cuda.Stream()
+
+    def images():
+        for q, p, spheres in zip(rs, pools, modes):
+            pv.copy_(p)
+            q.execute(pv, len(p), u, stream, sphereRenderFl=spheres)
+            last.execute(pv, len(p), u, stream, sphereRenderFl=spheres)
+        pv.zero_()
+
+    def check(what):
+        torch.cuda.synchronize()
+        for i, q in enumerate(rs):
+            for k, w in zip(("color", "depth"), want[i]):
+                same_bits(q.download(k), w, f"{what} {i} {k}")
+        for k, w in zip(("color", "depth"), want[-1]):
+            same_bits(last.download(k), w, f"{what} last {k}")
+
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        for _ in range(20):
+            images()
+    check("stream")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        images()
+    for q in rs + [last]:
+        q.execute(pv, 0, u)  # empties them
+    for _ in range(20):
+        graph.replay()
+    check("graph")
+    for q in rs + [last]:
+        q.close()

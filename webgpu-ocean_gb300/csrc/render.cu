@@ -44,12 +44,16 @@
 #include <vector>
 
 #include "../../include/mpm.h"
+#include "pdl.cuh"
 #include "render_math.cuh"
 
 namespace mpm {
 void set_last_error(const std::string& msg);  // capi.cu
 }
 
+using mpm::launch_pdl;
+using mpm::pdl_begin;
+using mpm::pdl_wait;
 using namespace mpm::rmath;
 
 namespace {
@@ -225,6 +229,7 @@ __global__ void __launch_bounds__(kBinBlock)
     k_tile_count(const float4* __restrict__ posvel, int first, int n, Uni u, Consts c, Bins bins,
                  unsigned long long* __restrict__ dkey, unsigned long long* __restrict__ tacc,
                  int npix) {
+    pdl_begin();
     extern __shared__ uint32_t s_count[];
     const int tiles = bins.tx * bins.ty;
     const int i = blockIdx.x * kBinBlock + threadIdx.x;
@@ -248,6 +253,8 @@ __global__ void __launch_bounds__(kBinBlock)
 
 // First entries of the tiles and the work items, one block.
 __global__ void __launch_bounds__(1024) k_tile_scan(Bins bins, uint32_t per) {
+    pdl_begin();
+    pdl_wait();
     constexpr uint32_t kOwn = 4;  // items of a tile that its thread writes
     __shared__ uint32_t s_w[2][32];
     const int tiles = bins.tx * bins.ty;
@@ -311,10 +318,12 @@ __global__ void __launch_bounds__(1024) k_tile_scan(Bins bins, uint32_t per) {
 
 // The tiles' entries.  A block reserves its share of each tile with one atomic.
 __global__ void __launch_bounds__(kBinBlock) k_tile_fill(int first, int n, Bins bins) {
+    pdl_begin();
     extern __shared__ uint32_t s_count[];
     const int tiles = bins.tx * bins.ty;
     for (int t = threadIdx.x; t < tiles; t += kBinBlock) s_count[t] = 0u;
     __syncthreads();
+    pdl_wait();
     const int i = blockIdx.x * kBinBlock + threadIdx.x;
     const uint32_t rect = i < n ? bins.rect[i] : kNoTile;
     uint32_t rank[4];
@@ -421,9 +430,11 @@ __global__ void __launch_bounds__(kTileBlock)
     __shared__ int s_item;
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const float radius = dvd(u.sphere_size, 2.0f);
-    const int items = bins.state[0], big = bins.state[1];
+    pdl_begin();
     if (THICK)
         for (int p = threadIdx.x; p < kTileCells; p += kTileBlock) s_lo[p] = s_hi[p] = 0u;
+    pdl_wait();
+    const int items = bins.state[0], big = bins.state[1];
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(bins.state + 2, 1);
         if (threadIdx.x < kTile) s_wide[threadIdx.x] = 0;
@@ -573,9 +584,10 @@ __global__ void __launch_bounds__(kTileBlock)
 }
 
 __global__ void k_resolve(const float4* __restrict__ posvel, Uni u, Consts c,
-                          const unsigned long long* __restrict__ dkey,
-                          const unsigned long long* __restrict__ tacc, float* __restrict__ depth,
-                          float* __restrict__ thick) {
+                          const unsigned long long* dkey, const unsigned long long* tacc,
+                          float* depth, float* thick) {
+    pdl_begin();
+    pdl_wait();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= c.W * c.H) return;
     const unsigned long long key = dkey[p];
@@ -683,7 +695,7 @@ struct Bilateral {
 
 template <bool X>
 __device__ __forceinline__ void bilateral_block(Bilateral<X>& sm, int block,
-                                                const float* __restrict__ src,
+                                                const float* src,
                                                 float* __restrict__ dst, const Consts& c,
                                                 const float* __restrict__ wtab) {
     constexpr int kW = Bilateral<X>::kW, kH = Bilateral<X>::kH;
@@ -756,7 +768,7 @@ struct Gaussian {
 
 template <bool X>
 __device__ __forceinline__ void gaussian_block(Gaussian<X>& sm, int block,
-                                               const float* __restrict__ src,
+                                               const float* src,
                                                float* __restrict__ dst, const Consts& c,
                                                const float* __restrict__ gtab) {
     constexpr int kTaps = 2 * kGaussFs + 1, kOut = 4;
@@ -837,6 +849,8 @@ template <bool X>
 __global__ void __launch_bounds__(kFilterThreads)
     k_filter(FilterPass depth, FilterPass thick, int depth_blocks, Consts c,
              const float* __restrict__ wtab, const float* __restrict__ gtab) {
+    pdl_begin();
+    pdl_wait();
     __shared__ __align__(16) union {
         Bilateral<X> bilateral;
         Gaussian<X> gaussian;
@@ -900,9 +914,11 @@ __device__ __forceinline__ V3 sample_cube(const float4* __restrict__ env, int si
               lerp2(c00.z, c10.z, c01.z, c11.z));
 }
 
-__global__ void k_shade(const float* __restrict__ depth_map, const float* __restrict__ thick_map,
+__global__ void k_shade(const float* depth_map, const float* thick_map,
                         const float4* __restrict__ env, int env_size, Uni u, Consts c,
                         float4* __restrict__ out, uchar4* __restrict__ out8) {
+    pdl_begin();
+    pdl_wait();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= c.W * c.H) return;
     const int px = p % c.W, py = p / c.W;
@@ -987,9 +1003,11 @@ __device__ __forceinline__ V3 value_to_color(float value) {
 }
 
 __global__ void k_sphere_shade(const float4* __restrict__ posvel, Uni u, Consts c,
-                               const unsigned long long* __restrict__ dkey,
+                               const unsigned long long* dkey,
                                float4* __restrict__ out, uchar4* __restrict__ out8,
                                float* __restrict__ depth) {
+    pdl_begin();
+    pdl_wait();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= c.W * c.H) return;
     const unsigned long long key = dkey[p];
@@ -1059,7 +1077,12 @@ bool binned(const mpm_renderer* r) { return (long long)r->bins.tx * r->bins.ty <
 // 20,000: 52 / 45 / 53, 70,000: 96 / 83 / 64, a million: 644 / 398 / 204).
 uint32_t item_size(int n) { return n < 10000 ? 32u : (n < 40000 ? 64u : (uint32_t)kItem); }
 
-// Clears the image's keys (and sums) and splats n particles into them.
+// Clears the image's keys (and sums) and splats n particles into them.  The
+// first launch is a plain one, the others of an image are let in early
+// (pdl.cuh): the gaps between the fluid view's 14 kernels, 1.5 to 2.5 us each,
+// were a tenth of an image's time.  Before and after, us: 70,000 particles as
+// spheres at 896x504 64.3 / 54.5, an application's frame of them with two
+// substeps 260.5 / 232.6, a million as a fluid at 1344x756 392 / 361.6.
 template <bool THICK>
 void enqueue_splats(mpm_renderer* r, const float4* pv, int n, const Uni& u, cudaStream_t st) {
     const Consts& c = r->c;
@@ -1081,12 +1104,10 @@ void enqueue_splats(mpm_renderer* r, const float4* pv, int n, const Uni& u, cuda
         const int cb = clear ? (clear + 4 * kBinBlock - 1) / (4 * kBinBlock) : 0;
         k_tile_count<<<blocks > cb ? blocks : cb, kBinBlock, smem, st>>>(pv, first, m, u, c, r->bins,
                                                                        r->dkey, tacc, clear);
-        k_tile_scan<<<1, 1024, 0, st>>>(r->bins, item_size(n));
-        k_tile_fill<<<blocks, kBinBlock, smem, st>>>(first, m, r->bins);
-        if (persp)
-            k_splat_tiles<THICK, true><<<r->tile_blocks[THICK][1], kTileBlock, 0, st>>>(pv, u, c, r->bins, r->dkey, tacc);
-        else
-            k_splat_tiles<THICK, false><<<r->tile_blocks[THICK][0], kTileBlock, 0, st>>>(pv, u, c, r->bins, r->dkey, tacc);
+        launch_pdl(k_tile_scan, 1, 1024, 0, st, r->bins, item_size(n));
+        launch_pdl(k_tile_fill, blocks, kBinBlock, smem, st, first, m, r->bins);
+        launch_pdl(persp ? k_splat_tiles<THICK, true> : k_splat_tiles<THICK, false>,
+                   r->tile_blocks[THICK][persp], kTileBlock, 0, st, pv, u, c, r->bins, r->dkey, tacc);
     }
 }
 
@@ -1258,7 +1279,7 @@ int mpm_renderer_execute(mpm_renderer* r, const void* posvel, int n,
     const int pb = (npix + 255) / 256;
     const float4* pv = static_cast<const float4*>(posvel);
     enqueue_splats<true>(r, pv, n, u, st);
-    k_resolve<<<pb, 256, 0, st>>>(pv, u, c, r->dkey, r->tacc, r->depth[0], r->thick[0]);
+    launch_pdl(k_resolve, pb, 256, 0, st, pv, u, c, r->dkey, r->tacc, r->depth[0], r->thick[0]);
     // blocks of w x h pixels, row by row (one grid dimension: images of one column have 2^28 rows)
     const auto grid = [&](int w, int h) { return (unsigned)((c.W + w - 1) / w) * (unsigned)((c.H + h - 1) / h); };
     const unsigned bx = grid(Bilateral<true>::kW, Bilateral<true>::kH);
@@ -1266,13 +1287,13 @@ int mpm_renderer_execute(mpm_renderer* r, const void* posvel, int n,
     for (int it = 0; it < 4; ++it) {  // fluidRender.ts:455-466, and once :474-486
         const unsigned gx = it ? 0u : grid(Gaussian<true>::kW, Gaussian<true>::kH);
         const unsigned gy = it ? 0u : grid(Gaussian<false>::kW, Gaussian<false>::kH);
-        k_filter<true><<<bx + gx, kFilterThreads, 0, st>>>({r->depth[0], r->depth[1]}, {r->thick[0], r->thick[1]},
-                                                          (int)bx, c, r->wtab, r->gtab);
-        k_filter<false><<<by + gy, kFilterThreads, 0, st>>>({r->depth[1], r->depth[0]}, {r->thick[1], r->thick[0]},
-                                                           (int)by, c, r->wtab, r->gtab);
+        launch_pdl(k_filter<true>, bx + gx, kFilterThreads, 0, st, FilterPass{r->depth[0], r->depth[1]},
+                   FilterPass{r->thick[0], r->thick[1]}, (int)bx, c, r->wtab, r->gtab);
+        launch_pdl(k_filter<false>, by + gy, kFilterThreads, 0, st, FilterPass{r->depth[1], r->depth[0]},
+                   FilterPass{r->thick[1], r->thick[0]}, (int)by, c, r->wtab, r->gtab);
     }
-    k_shade<<<pb, 256, 0, st>>>(r->depth[0], r->thick[0], r->env, r->env_size, u, c, r->color,
-                                r->color8);
+    launch_pdl(k_shade, pb, 256, 0, st, r->depth[0], r->thick[0], r->env, r->env_size, u, c, r->color,
+               r->color8);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "mpm_renderer_execute");
     return MPM_OK;
@@ -1289,7 +1310,7 @@ int mpm_renderer_execute_spheres(mpm_renderer* r, const void* posvel, int n,
     const int pb = (npix + 255) / 256;
     const float4* pv = static_cast<const float4*>(posvel);
     enqueue_splats<false>(r, pv, n, u, st);
-    k_sphere_shade<<<pb, 256, 0, st>>>(pv, u, c, r->dkey, r->color, r->color8, r->depth[0]);
+    launch_pdl(k_sphere_shade, pb, 256, 0, st, pv, u, c, r->dkey, r->color, r->color8, r->depth[0]);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "mpm_renderer_execute_spheres");
     return MPM_OK;
