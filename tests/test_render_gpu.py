@@ -287,6 +287,30 @@ def test_filters(cuda, pkg, oracle_mod, W, H, radius, dist):
     r.close()
 
 
+@pytest.mark.parametrize("radius,gap", [(0.6, 28.0), (0.5, 23.5)])  # a divisor that is a power of two, one that is not
+def test_filters_across_depth_gaps(cuda, pkg, oracle_mod, radius, gap):
+    """Neighbouring pixels whose depths differ so much that the weights are
+    subnormal, down to where they are 0 (quotients from -87 to -105)."""
+    import torch
+    W, H = 131, 99
+    rng = np.random.default_rng(8)
+    target = np.array([10.0, 4.0, 12.0])
+    u = pkg.camera_uniforms(W, H, 45.0, list(target), FOV, 0.6)
+    right, up, back = np.array(u.view_matrix[:]).reshape(4, 4)[:3, :3].T  # the camera's axes
+    # two sheets along the view, one behind the other by gap, give or take a twentieth
+    behind = np.where(rng.random(3000) < 0.5, 0.0, gap * (1.0 + 0.1 * (rng.random(3000) - 0.5)))
+    across = (rng.random((3000, 2)) - 0.5) * 40.0
+    pv = np.zeros((3000, 8), np.float32)
+    pv[:, 0:3] = target + across[:, :1] * right + across[:, 1:] * up - behind[:, None] * back
+    r = pkg.FluidRenderer(W, H, radius, FOV)
+    dev = torch.from_numpy(pv).cuda()
+    r.execute(dev, len(pv), u)
+    want = oracle_mod.render(pv, uniforms_f32(u), W, H, radius, FOV, default_env_from(pkg))
+    for k in ("depth", "thickness", "color", "color8"):
+        same_bits(r.download(k), want[k], k)
+    r.close()
+
+
 def test_images_in_a_row(cuda, pkg):
     """An image's launches overlap one another, not what stands before and
     after them in the stream: images behind writes of their particles, on a

@@ -14,44 +14,12 @@
 // p2g1_particle, p2g2_particle and g2p_particle in mpm_math.cuh, which the
 // tests check.
 #pragma once
+#include "f32x2.cuh"
 #include "mpm_math.cuh"
 
 namespace mpm {
 
-struct f2 {
-    unsigned long long v;
-};
-
-__device__ __forceinline__ f2 pk(float a, float b) {
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void upk(f2 x, float& a, float& b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
-}
-__device__ __forceinline__ float lo(f2 x) {
-    float a, b;
-    upk(x, a, b);
-    return a;
-}
-__device__ __forceinline__ float hi(f2 x) {
-    float a, b;
-    upk(x, a, b);
-    return b;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-    f2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
-    return d;
-}
-// Only for operands that are not packed products (see the file comment).
-__device__ __forceinline__ f2 add2(f2 a, f2 b) {
-    f2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
-    return d;
-}
-__device__ __forceinline__ f2 dup(float a) { return pk(a, a); }
+using namespace x2;
 
 // p2g_1.wgsl:24-65.  sink(gx, gy, gz, m, vx, vy, vz) with i32 values.
 template <class Sink>

@@ -41,9 +41,11 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/mpm.h"
+#include "f32x2.cuh"
 #include "pdl.cuh"
 #include "render_math.cuh"
 
@@ -51,6 +53,7 @@ namespace mpm {
 void set_last_error(const std::string& msg);  // capi.cu
 }
 
+using namespace mpm::x2;
 using mpm::launch_pdl;
 using mpm::pdl_begin;
 using mpm::pdl_wait;
@@ -643,26 +646,67 @@ __global__ void k_weight_tables(float* __restrict__ wtab, float* __restrict__ gt
     }
 }
 
-// exp_r(a / b) for a <= 0 and the filter's b = two_sd, the same bits with
+// exp_series() of two numbers.  A packed product that only a packed sum reads
+// would become one fused operation of other rounding; a fused one with
+// -0 to add rounds as the product does and stays as it is.
+__device__ __forceinline__ f2 exp_series2(f2 r, f2 zero) {
+    f2 p = dup(2.48015873e-5f);
+    p = add2(fma2(p, r, zero), dup(1.98412698e-4f));
+    p = add2(fma2(p, r, zero), dup(1.38888889e-3f));
+    p = add2(fma2(p, r, zero), dup(8.33333333e-3f));
+    p = add2(fma2(p, r, zero), dup(4.16666667e-2f));
+    p = add2(fma2(p, r, zero), dup(1.66666667e-1f));
+    p = add2(fma2(p, r, zero), dup(0.5f));
+    p = add2(fma2(p, r, zero), dup(1.0f));
+    p = add2(fma2(p, r, zero), dup(1.0f));
+    return p;
+}
+
+// exp_r(a / b) for a = -d^2 <= 0 and the filter's b = two_sd, the same bits with
 // fewer operations and no branch, so that the taps of a pixel overlap.  The
 // quotient: a product with 1 / b where b is a power of two (the application's
 // radius: 8), else quot() with RN(1 / b); quotients too small for quot() give
 // exp = 1 either way.  The rounding of x / ln 2 by an addition that leaves only
-// the integer.
+// the integer k, and 2^k as 2^(k + 64) * 2^-64: for k in [-152, 0] the first
+// product is exact, so the result is rounded once, as exp_r's is.
 struct DepthWeight {
     float b, rb, cut;  // cut: below it a / b < -104 and the weight is 0
     bool range, pow2;  // b fits quot(), is a power of two
     template <bool POW2>
-    __device__ __forceinline__ float at(float a) const {
+    __device__ __forceinline__ float at(float d) const {
+        const float a = mul(-d, d);
         const float x = POW2 ? mul(a, rb) : quot(a, b, rb);
-        const float magic = 12582912.0f;  // 1.5 * 2^23
-        const float shifted = add(mul(x, 1.44269502f), magic);
-        const int k = __float_as_int(shifted) - 0x4b400000;
-        const float kf = sub(shifted, magic);
+        const float shifted = add(mul(x, 1.44269502f), kMagic);
+        const float kf = sub(shifted, kMagic);
         const float r = sub(sub(x, mul(kf, 0.693145751953125f)), mul(kf, 1.42860677e-6f));
-        const int k1 = k >> 1;
-        const float e = mul(mul(exp_series(r), pow2i(k1)), pow2i(k - k1));
+        const float e = mul(mul(exp_series(r), scale(shifted)), 0x1p-64f);
         return a < cut ? 0.0f : e;
+    }
+    // Two of them, in packed operations.
+    template <bool POW2>
+    __device__ __forceinline__ f2 at2(f2 d, f2 zero) const {
+        const f2 a = mul2(d, neg2(d));
+        f2 x;
+        if (POW2) {
+            x = mul2(a, dup(rb));
+        } else {
+            const f2 nb = dup(-b), y = dup(rb);
+            x = mul2(a, y);
+            x = fma2(fma2(nb, x, a), y, x);
+            x = fma2(fma2(nb, x, a), y, x);
+        }
+        const f2 shifted = add2(fma2(x, dup(1.44269502f), zero), dup(kMagic));
+        const f2 kf = add2(shifted, dup(-kMagic));
+        f2 r = add2(x, fma2(kf, dup(-0.693145751953125f), zero));
+        r = add2(r, fma2(kf, dup(-1.42860677e-6f), zero));
+        const f2 scales = pk(scale(lo(shifted)), scale(hi(shifted)));
+        const f2 e = mul2(mul2(exp_series2(r, zero), scales), dup(0x1p-64f));
+        return pk(lo(a) < cut ? 0.0f : lo(e), hi(a) < cut ? 0.0f : hi(e));
+    }
+    static constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
+    // 2^(k + 64) from k + kMagic
+    static __device__ __forceinline__ float scale(float shifted) {
+        return __int_as_float((__float_as_int(shifted) << 23) + (191 << 23));
     }
 };
 
@@ -678,12 +722,18 @@ __device__ __forceinline__ DepthWeight depth_weight(const Consts& c) {
 }
 
 // One pass of the separable bilateral filter [bilateral.wgsl:18-75], along x
-// (X) or y.  Bound by the chain of a tap's exp and by the start of its short
-// launches.  A block holds the depths that its taps reach, as far as its widest
-// filter, clamped to the image, in shared memory, so that a tap has no index
-// arithmetic, and the taps' weights have no branch, so that several overlap.
-// Per pass (ncu) at 896x504 15.5 -> 12.0 us, at 1344x756 20.9 -> 16.8 us;
-// shared memory alone 13.3 and 18.3.
+// (X) or y.  Bound by the issue of the taps' exp and, where the filters are
+// short, by the start of its launches.  A block holds the depths that its taps
+// reach, as far as its widest filter, clamped to the image, in shared memory, so
+// that a tap has no index arithmetic, and the taps' weights have no branch and
+// are made two at a time.  Per pass (ncu) at 896x504 15.5 -> 12.0 us, at 1344x756
+// 20.9 -> 16.8 us before the pairs; shared memory alone 13.3 and 18.3.  A pair's
+// packed operations, whole images: 70,000 particles at 896x504 152.5 -> 145.5 us,
+// from half as far 566 -> 534, 200,000 at 1200x800 683 -> 639, a million at
+// 1344x756 364 -> 355.  One pair at a time: with the loop unrolled to two or four
+// 151 / 146, 549 / 531, 652 / 646, 354 / 362.  Loading the first few texels of the
+// halo together with the pixels' own, before the filters' widths are known: no
+// faster.
 constexpr int kFilterThreads = 256;
 
 template <bool X>
@@ -734,20 +784,32 @@ __device__ __forceinline__ void bilateral_block(Bilateral<X>& sm, int block,
     const float* wrow = wtab + fs * kWRow;
     const DepthWeight weight = depth_weight(c);
     float sum = 0.0f, wsum = 0.0f;
-    auto walk = [&](auto&& weight_of) {
-#pragma unroll 4
-        for (int x = -fs; x <= fs; ++x) {
-            const float sampled = tap[X ? x : x * kW];
-            const float rd = sub(sampled, depth);
-            const float w = __ldg(wrow + (x < 0 ? -x : x));
-            const float wd = weight_of(mul(-rd, rd));
-            sum = add(sum, mul(mul(sampled, w), wd));
-            wsum = add(wsum, mul(w, wd));
-        }
+    auto term = [&](float sampled, float w, float wd) {
+        sum = add(sum, mul(mul(sampled, w), wd));
+        wsum = add(wsum, mul(w, wd));
     };
-    if (weight.range && weight.pow2) walk([&](float a) { return weight.template at<true>(a); });
-    else if (weight.range) walk([&](float a) { return weight.template at<false>(a); });
-    else walk([&](float a) { return exp_r(dvd(a, weight.b)); });
+    auto at = [&](int x) { return tap[X ? x : x * kW]; };
+    auto spatial = [&](int x) { return __ldg(wrow + (x < 0 ? -x : x)); };
+    auto walk = [&](auto pow2) {
+        constexpr bool POW2 = decltype(pow2)::value;
+        const f2 nd = dup(-depth), zero = negative_zeros(c.W);
+#pragma unroll 1
+        for (int x = -fs; x < fs; x += 2) {
+            const f2 sampled = pk(at(x), at(x + 1)), w = pk(spatial(x), spatial(x + 1));
+            const f2 wd = weight.template at2<POW2>(add2(sampled, nd), zero);
+            const f2 sw = mul2(mul2(sampled, w), wd), ww = mul2(w, wd);
+            sum = add(add(sum, lo(sw)), hi(sw));
+            wsum = add(add(wsum, lo(ww)), hi(ww));
+        }
+        term(at(fs), spatial(fs), weight.template at<POW2>(sub(at(fs), depth)));
+    };
+    if (weight.range && weight.pow2) walk(std::true_type{});
+    else if (weight.range) walk(std::false_type{});
+    else
+        for (int x = -fs; x <= fs; ++x) {
+            const float rd = sub(at(x), depth);
+            term(at(x), spatial(x), exp_r(dvd(mul(-rd, rd), weight.b)));
+        }
     dst[p] = dvd(sum, wsum);
 }
 
