@@ -19,10 +19,10 @@
 //  * A task is one bin's particles, or the particles of both bins of a z
 //    pair (4x4x8 cells) when together they number at most Dev::pair_max (a
 //    runtime parameter, autotuned: sparse bricks then share one task's fixed
-//    costs).  CTAs claim tasks from an atomic work counter and walk a task in
-//    chunks of one particle per thread.  In tasks
-//    of at least Dev::lane_min particles (a runtime parameter, autotuned),
-//    p2g_2 first reorders the bin's particles into a lane table that puts
+//    costs).  CTAs take their first two tasks by their number, claim the
+//    others from an atomic work counter, and walk a task in chunks of one
+//    particle per thread.  In tasks of at least Dev::lane_min particles (a
+//    runtime parameter, autotuned), p2g_2 first reorders the bin's particles into a lane table that puts
 //    particles of 32 different shared-memory bank classes in the 32 lanes of
 //    a warp (build_lane_table); g2p reuses that order.  The CTA keeps the
 //    cells the task's stencils reach (its "arena") in shared memory: the
@@ -183,7 +183,7 @@ struct Dev {
     uint32_t* rank_of;
     uint32_t* bin_count;  // [bins + 1]
     uint32_t* bin_start;  // [bins + 2]
-    uint32_t* chunk_sum;  // [3 * chunks]: per 1024 bins, particles and multi-/single-chunk tasks
+    uint32_t* chunk_sum;  // [3 * chunks]: per kScanThreads bins, particles and multi-/single-chunk tasks
     uint32_t* order;
     Task* tasks;          // [task_slots]: multi-chunk tasks from the front, the others from the back
     uint32_t* ntasks;     // [2]: all tasks, multi-chunk tasks
@@ -1077,10 +1077,11 @@ __global__ void __launch_bounds__(kTask) k_bin(Particles P, Scene one, Dev d, in
 // per non-empty bin, or several when it holds more than task_cap particles;
 // tasks of more than one chunk are stored from the front of the list, the
 // others from the back (task_slot).  one_g is a single scene's geometry;
-// batches read theirs from the table.  CTA c scans bins [c*1024,
-// (c+1)*1024); it finds its starting offsets by reducing all earlier counts
-// itself (a few KB to a few hundred KB from L2), so no CTA waits on another.
-// The counts are zeroed by k_scatter, which runs next.
+// batches read theirs from the table.  CTA c scans
+// kScanThreads bins from c*kScanThreads; it finds its starting offsets by
+// reducing all earlier counts itself, from L2, or k_chunk_sums' sums where
+// there are many, so no CTA waits on another.  The counts are zeroed by
+// k_scatter, which runs next.
 
 constexpr int kScanWarps = kScanThreads / 32;
 
