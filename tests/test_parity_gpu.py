@@ -559,6 +559,28 @@ def test_scan_chunk_edges(cuda, pkg, oracle_mod, box):
     sim.close()
 
 
+@pytest.mark.parametrize("box", [(124, 44, 48), (64, 64, 64)])
+def test_scan_and_scatter_in_one_launch(cuda, pkg, oracle_mod, box):
+    """Either side of the most bins (4,096) that are scanned and scattered in
+    one launch (4,094 and 4,098 bins), particle counts around a block's share,
+    and frames that time every stage, which launch the two apart, between
+    frames that do not."""
+    rng = np.random.default_rng(box[0])
+    for n in (1, 1023, 1025, 7000):
+        recs = np.zeros((n, 20), np.float32)
+        recs[:, 0:3] = 2.0 + rng.random((n, 3)) * (np.array(box) - 4.5)
+        recs[:, 4:7] = rng.normal(0.0, 0.5, (n, 3))
+        sim = make_sim(pkg, "sorted", max_particles=7000, max_grid=box)
+        sim.upload(recs, [float(b) for b in box])
+        ref = oracle_mod.OracleSim(sim.downloadParticles(), [float(b) for b in box])
+        for profiled in (False, True, True, False, False):
+            sim.setProfiling(profiled)
+            sim.execute()
+            ref.execute(2, NTHREADS)
+        assert_state_equal(sim, ref, f"box {box} n {n}")
+        sim.close()
+
+
 def test_constants_that_change_between_calls(cuda, pkg, oracle_mod):
     """Calls that keep the constants replay a graph, calls that change them
     launch their kernels: walls moving every frame, resting, moving while
