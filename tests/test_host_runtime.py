@@ -1,0 +1,58 @@
+"""The library's host side over a CUDA runtime that runs no kernels
+(fake_cudart.cpp): what it launches, what it waits for, and what it does when
+memory is short.  On CPU."""
+from __future__ import annotations
+
+import ctypes
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+SIDE_STREAM = 0x1000  # a stream of the caller's own, as a handle
+
+
+@pytest.fixture(scope="session")
+def fake_lib(pkg, tmp_path_factory):
+    """Path of the library with the fake runtime."""
+    nvcc = shutil.which(pkg.build.nvcc())
+    objects = [os.path.join(pkg.build.BUILD, src.replace(".cu", ".o")) for src in pkg.build.SOURCES]
+    if not (nvcc and shutil.which("g++")):
+        pytest.skip("no host toolchain")
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
+    out = str(tmp_path_factory.mktemp("fake") / "libmpm_fake.so")
+    subprocess.check_call(["g++", "-shared", "-fPIC", "-std=c++17", "-O1", "-I" + cuda, "-Wl,-Bsymbolic",
+                           "-Wl,-z,defs", "-o", out, os.path.join(HERE, "fake_cudart.cpp"), *objects])
+    return out
+
+
+@pytest.fixture
+def fake(pkg, fake_lib, monkeypatch):
+    """The package over that library; fake.fake_*: the runtime's own functions."""
+    monkeypatch.setattr(pkg._lib, "_lib", None)
+    monkeypatch.setattr(pkg.build, "build", lambda *a, **k: fake_lib)
+    lib = pkg._lib.load()
+    lib.fake_reset.argtypes = [ctypes.c_size_t]
+    lib.fake_largest.restype = ctypes.c_size_t
+    lib.fake_launched.restype = ctypes.c_char_p
+    lib.fake_reset(-1)
+    return lib
+
+
+def test_sph_upload_is_done_when_it_returns(fake, pkg):
+    """A frame on the caller's own stream does not wait for the null stream, so
+    the upload's copies and memsets have to be done when it returns."""
+    sim = pkg.SPHSimulator(None, None, 0.08, maxParticles=100)
+    recs = np.zeros((100, 16), np.float32)
+    for graph in (False, True):
+        sim.setGraph(graph)
+        sim.upload(recs, [1.0, 2.0, 1.0])
+        sim.execute(SIDE_STREAM)
+        sim.reset(100, [1.0, 2.0, 1.0])
+        sim.execute(SIDE_STREAM)
+    assert b"k_sph_force" in fake.fake_launched()
+    assert fake.fake_unordered() == 0
+    sim.close()

@@ -198,3 +198,21 @@ def test_sph_solver_reproduces_wgsl_golden(cuda, pkg, name):
         assert_bits_equal(sim.downloadParticles(), f[f"s{s}_particles"], f"{name} substep {s}")
         assert_bits_equal(sim.downloadPosvel(), f[f"s{s}_posvel"], f"{name} substep {s} posvel")
     sim.close()
+
+
+def test_frames_on_a_side_stream_after_an_upload(cuda, pkg, oracle_mod):
+    """A frame on a stream of the caller's own finds the upload done: the
+    records of particles outside the grid, which the frame's first kernel
+    writes, are not overwritten by what the upload clears."""
+    recs = pkg.sph_scene_dambreak([1.0, 2.0, 1.0], 30000, 3)
+    recs[::7, 1] = -3.0
+    recs[::7, 4:7] = 0.25
+    sim = pkg.SPHSimulator(None, None, 0.08, maxParticles=len(recs))
+    stream = cuda.cuda.Stream()
+    want, pv = oracle_mod.sph_execute(recs, [1.0, 2.0, 1.0], 2)
+    for _ in range(10):
+        sim.upload(recs, [1.0, 2.0, 1.0])
+        sim.execute(stream)
+        assert_bits_equal(sim.downloadParticles(), want, "records")
+        assert_bits_equal(sim.downloadPosvel(), pv, "posvel")
+    sim.close()

@@ -977,6 +977,9 @@ int mpm_sph_upload(mpm_sph* s, const float* rec64, int n, const float real_half[
     if (n && err == cudaSuccess) err = cudaMemcpy(s->V, V.data(), sizeof(float4) * n, cudaMemcpyHostToDevice);
     if (n && err == cudaSuccess) err = cudaMemcpy(s->F, F.data(), sizeof(float4) * n, cudaMemcpyHostToDevice);
     if (n && err == cudaSuccess) err = cudaMemset(s->posvel, 0, sizeof(float4) * 2 * (size_t)n);
+    // copies from pageable memory and memsets may outlast their calls, and a
+    // frame on a non-blocking stream would not wait for them
+    if (err == cudaSuccess) err = cudaDeviceSynchronize();
     if (err != cudaSuccess) return cuda_fail(err, "mpm_sph_upload");
     s->n = n;
     for (int a = 0; a < 3; ++a) s->real_half[a] = real_half[a];
