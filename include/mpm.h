@@ -434,7 +434,11 @@ void* mpm_renderer_color_device_ptr(mpm_renderer* renderer);
  * SPHSimulator.reset/changeBoxSize take them. */
 typedef struct mpm_sph mpm_sph;
 
-/* constructor(particleBuffer, posvelBuffer, renderDiameter, device), sph.ts:46 */
+/* constructor(particleBuffer, posvelBuffer, renderDiameter, device), sph.ts:46.
+ * Device memory per particle of capacity: 140 bytes (172 with a posvel buffer
+ * of its own), and up to 2^23 particles 512 more for neighbour lists; where
+ * there is no room for those the frames run without, slower, with the same
+ * results. */
 int mpm_sph_create(int max_particles, float render_diameter, void* posvel_device,
                    size_t posvel_bytes, mpm_sph** out);
 int mpm_sph_destroy(mpm_sph* sph);

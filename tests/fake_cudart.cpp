@@ -18,8 +18,9 @@
 
 namespace {
 
-size_t g_most = ~(size_t)0;  // bytes of one allocation
-size_t g_largest = 0;        // granted so far
+size_t g_room = ~(size_t)0;  // bytes of device memory
+size_t g_used = 0;
+std::map<void*, size_t> g_size;
 cudaError_t g_error = cudaSuccess;
 bool g_pending = false;      // null-stream work that nothing has waited for
 int g_unordered = 0;
@@ -64,16 +65,15 @@ cudaError_t gone(T handle) {
 
 extern "C" {
 
-void fake_reset(size_t most) {
-    g_most = most;
-    g_largest = 0;
+void fake_reset(size_t room) {
+    g_room = room;
     g_error = cudaSuccess;
     g_pending = false;
     g_unordered = 0;
     g_launched.clear();
 }
 int fake_unordered() { return g_unordered; }
-size_t fake_largest() { return g_largest; }
+size_t fake_used() { return g_used; }
 const char* fake_launched() { return g_launched.c_str(); }
 
 void** __cudaRegisterFatBinary(void*) { return reinterpret_cast<void**>(&g_config); }
@@ -108,12 +108,19 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void
 
 cudaError_t cudaMalloc(void** p, size_t bytes) {
     *p = nullptr;
-    if (bytes > g_most) return result(cudaErrorMemoryAllocation);
-    if (bytes > g_largest) g_largest = bytes;
+    if (bytes > g_room - g_used) return result(cudaErrorMemoryAllocation);
     *p = std::calloc(bytes ? bytes : 1, 1);  // pages that nothing touches take no room
-    return result(*p ? cudaSuccess : cudaErrorMemoryAllocation);
+    if (!*p) return result(cudaErrorMemoryAllocation);
+    g_used += bytes;
+    g_size[*p] = bytes;
+    return cudaSuccess;
 }
-cudaError_t cudaFree(void* p) { std::free(p); return cudaSuccess; }
+cudaError_t cudaFree(void* p) {
+    g_used -= g_size[p];
+    g_size.erase(p);
+    std::free(p);
+    return cudaSuccess;
+}
 cudaError_t cudaMallocAsync(void** p, size_t bytes, cudaStream_t) { return cudaMalloc(p, bytes); }
 cudaError_t cudaFreeAsync(void* p, cudaStream_t) { return cudaFree(p); }
 

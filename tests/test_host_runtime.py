@@ -36,7 +36,7 @@ def fake(pkg, fake_lib, monkeypatch):
     monkeypatch.setattr(pkg.build, "build", lambda *a, **k: fake_lib)
     lib = pkg._lib.load()
     lib.fake_reset.argtypes = [ctypes.c_size_t]
-    lib.fake_largest.restype = ctypes.c_size_t
+    lib.fake_used.restype = ctypes.c_size_t
     lib.fake_launched.restype = ctypes.c_char_p
     lib.fake_reset(-1)
     return lib
@@ -56,3 +56,25 @@ def test_sph_upload_is_done_when_it_returns(fake, pkg):
     assert b"k_sph_force" in fake.fake_launched()
     assert fake.fake_unordered() == 0
     sim.close()
+
+
+def test_sph_without_room_for_neighbour_lists(fake, pkg):
+    """2^23 particles, the most with neighbour lists: 4.3 GB of them beside 1.5
+    GB.  Where they do not fit the simulator works without; where the rest does
+    not fit either, creating it fails and leaves nothing behind."""
+    cap = 1 << 23
+    sim = pkg.SPHSimulator(None, None, 0.08, maxParticles=cap)
+    assert fake.fake_used() > 512 * cap
+    sim.close()
+    assert fake.fake_used() == 0
+    fake.fake_reset(2 << 30)
+    sim = pkg.SPHSimulator(None, None, 0.08, maxParticles=cap)
+    assert fake.fake_used() < 2 << 30
+    sim.upload(np.zeros((1000, 16), np.float32), [1.0, 2.0, 1.0])
+    sim.execute()
+    assert b"k_sph_force" in fake.fake_launched()
+    sim.close()
+    fake.fake_reset(1 << 30)
+    with pytest.raises(pkg.MPMError):
+        pkg.SPHSimulator(None, None, 0.08, maxParticles=cap)
+    assert fake.fake_used() == 0

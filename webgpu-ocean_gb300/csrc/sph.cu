@@ -403,7 +403,7 @@ __device__ __forceinline__ void neighbour_row(const Env& e, const unsigned* __re
 // bottom's did, 400,000 particles 1165 instead of 758 us).  Entry k of sorted
 // particle s is nbr[k * stride + s], so that neighbouring particles' entries
 // share sectors.  No lists are kept for capacities above kListedMax, where
-// they would take over 4 GB.
+// they would take over 4 GB, nor where there is no memory for them.
 constexpr int kNeighbours = 128;
 constexpr int kListedMax = 1 << 23;
 
@@ -909,6 +909,7 @@ int mpm_sph_create(int max_particles, float render_diameter, void* posvel_device
     // much as a frame), each at a 256-byte boundary; twice through the list:
     // once for the size, once for the places
     size_t bytes = 0;
+    bool lists = np <= kListedMax;
     auto place = [&](auto& ptr, size_t count) {
         if (s->slab) ptr = reinterpret_cast<std::remove_reference_t<decltype(ptr)>>(s->slab + bytes);
         bytes += (sizeof(*ptr) * count + 255) / 256 * 256;
@@ -927,24 +928,33 @@ int mpm_sph_create(int max_particles, float render_diameter, void* posvel_device
         place(s->chunk, kMaxChunks);
         place(s->start, cells);
         place(s->box_d, 3);
-        if (np <= kListedMax) place(s->nl.nbr, kNeighbours * np);
+        if (lists) place(s->nl.nbr, kNeighbours * np);
     };
     s->nl.stride = np;
-    place_all();
-    cudaError_t err = cudaMalloc(&s->slab, bytes);
+    cudaError_t err = cudaSuccess;
+    if (posvel_device) {
+        s->posvel = static_cast<float4*>(posvel_device);
+    } else {
+        s->posvel_owned = true;
+        err = cudaMalloc(&s->posvel, sizeof(float4) * 2 * np);
+    }
+    if (err == cudaSuccess) {
+        place_all();
+        err = cudaMalloc(&s->slab, bytes);
+    }
+    if (err == cudaErrorMemoryAllocation && s->posvel && lists) {
+        // the lists are most of it, and the simulator does without
+        cudaGetLastError();
+        s->slab = nullptr;
+        lists = false;
+        place_all();
+        err = cudaMalloc(&s->slab, bytes);
+    }
     if (err == cudaSuccess) {
         place_all();
         // zero between substeps: the scan and the scatter clear what they have read
         err = cudaMemset(s->count, 0, 4 * cells);
         if (err == cudaSuccess) err = cudaMemset(s->chunk, 0, 4 * kMaxChunks);
-    }
-    if (err == cudaSuccess) {
-        if (posvel_device) {
-            s->posvel = static_cast<float4*>(posvel_device);
-        } else {
-            err = cudaMalloc(&s->posvel, sizeof(float4) * 2 * np);
-            s->posvel_owned = true;
-        }
     }
     if (err != cudaSuccess) {
         const int rc = cuda_fail(err, "mpm_sph_create");
