@@ -452,11 +452,12 @@ int mpm_sph_step(mpm_sph* sph, int substeps, void* stream);
 /* Frames replay as CUDA graphs (captured once per substep and particle
  * count); 0 launches every kernel each frame.  Results are the same. */
 int mpm_sph_set_graph(mpm_sph* sph, int enable); /* default 1 */
-/* Up to max_particles particles, the forces may run with several lanes of a
- * warp per particle, and do where that is the faster way (the lanes share
- * the neighbour terms; the sums keep the one-thread order, so the results do
- * not change); above it, one thread per particle.  Default 32768; 0: always
- * a thread per particle; -1: the default. */
+/* Up to max_particles particles, density and forces run with 8 or 16 lanes of
+ * a warp per particle (the lanes share the neighbour terms; the sums keep the
+ * one-thread order, so the results do not change); above it, one thread per
+ * particle.  0: always a thread per particle; -1 or 32768, which is what the
+ * default reads as: the faster at each particle count (lanes up to 22,000
+ * particles for the forces, up to 130,000 for the densities). */
 int mpm_sph_set_warp_per_particle(mpm_sph* sph, int max_particles);
 int mpm_sph_get_warp_per_particle(const mpm_sph* sph);
 /* changeBoxSize(realBoxSize), sph.ts:383-388 (half sizes) */

@@ -78,3 +78,27 @@ def test_sph_without_room_for_neighbour_lists(fake, pkg):
     with pytest.raises(pkg.MPMError):
         pkg.SPHSimulator(None, None, 0.08, maxParticles=cap)
     assert fake.fake_used() == 0
+
+
+@pytest.mark.parametrize("n,warp_max,density,force", [
+    (12000, -1, 16, 16), (12001, -1, 8, 8), (22000, -1, 8, 8), (22001, -1, 8, 1),
+    (130000, -1, 8, 1), (130001, -1, 1, 1),
+    (1, 0, 1, 1), (12000, 0, 1, 1), (100000, 0, 1, 1),          # 0: always a thread
+    (500, 500, 16, 16), (501, 500, 1, 1),                       # the caller's own limit
+    (30000, 32767, 8, 8), (30000, 32768, 8, 1), (30000, 29999, 1, 1), (140000, 200000, 8, 8),
+])
+def test_sph_lanes_per_particle(fake, pkg, n, warp_max, density, force):
+    """Which kernels run: the fastest at a particle count, or the ones that the
+    caller's limit asks for, of the densities and of the forces."""
+    sim = pkg.SPHSimulator(None, None, 0.08, maxParticles=n)
+    sim.setGraph(False)
+    sim.upload(np.zeros((n, 16), np.float32), [1.0, 2.0, 1.0])
+    sim.warpPerParticle = warp_max
+    sim.execute(substeps=1)
+    ran = fake.fake_launched().decode()
+    for what, lanes in (("density", density), ("force", force)):
+        name = f"k_sph_{what}_thread" if lanes == 1 else f"k_sph_{what}ILi{lanes}E"
+        assert [k for k in ran.split() if f"k_sph_{what}" in k] == [k for k in ran.split() if name in k] != []
+    sim.warpPerParticle = -1
+    assert sim.warpPerParticle == 32768
+    sim.close()

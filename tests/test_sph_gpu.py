@@ -216,3 +216,23 @@ def test_frames_on_a_side_stream_after_an_upload(cuda, pkg, oracle_mod):
         assert_bits_equal(sim.downloadParticles(), want, "records")
         assert_bits_equal(sim.downloadPosvel(), pv, "posvel")
     sim.close()
+
+
+@pytest.mark.parametrize("capacity", [5000, (1 << 23) + 1])  # with neighbour lists, without
+@pytest.mark.parametrize("n", [1, 31, 33, 127, 129, 5000])
+def test_a_thread_per_particle(cuda, pkg, oracle_mod, n, capacity):
+    """The one-thread kernels at counts around their warps and blocks: a fall
+    of ten frames, some particles outside the grid or aliasing into it."""
+    recs = pkg.sph_scene_dambreak([0.5, 2.0, 0.5], n, 3)
+    odd = np.array([[0.0, -3.0, 0.0], [5.0, 0.0, 0.0], [-2.2, 0.1, 0.1], [0.0, 2.3, 0.0],
+                    [np.nan, 0.0, 0.0], [1e30, -1e30, 0.0]], np.float32)
+    m = min(len(odd), n // 5)
+    recs[:m, 0:3] = odd[:m]
+    sim = pkg.SPHSimulator(None, None, 0.08, maxParticles=capacity)
+    sim.warpPerParticle = 0
+    sim.upload(recs, [0.5, 2.0, 0.5])
+    for _ in range(10):
+        sim.execute()
+        recs, pv = oracle_mod.sph_execute(recs, [0.5, 2.0, 0.5], 2)
+    assert_bits_equal(sim.downloadParticles(), recs, "records")
+    sim.close()

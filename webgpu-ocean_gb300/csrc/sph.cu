@@ -797,8 +797,7 @@ struct SplitMix64 {
 constexpr int kSph16Max = 12000;
 constexpr int kSphLanesMax = 22000;
 constexpr int kSphDensity8Max = 130000;
-// Default of mpm_sph::warp_max: particle counts above it run no group of lanes
-// for the forces, whatever the limits above allow.
+// The limit on particle counts with lanes, as long as the counts above decide.
 constexpr int kSphWarpMaxDefault = 32768;
 
 struct mpm_sph {
@@ -825,7 +824,7 @@ struct mpm_sph {
     float* box_d = nullptr;
     float box_uploaded[3] = {NAN, NAN, NAN};
     bool graph = true;
-    int warp_max = kSphWarpMaxDefault;  // see above
+    int warp_max = -1;  // lanes per particle up to this count, a thread above; -1: see above
     struct FrameGraph {
         int substeps, n;
         cudaGraphExec_t exec;
@@ -1085,18 +1084,15 @@ void enqueue_substeps(mpm_sph* s, int substeps, cudaStream_t st) {
         // over n, the most there can be
         k_sph_place<<<pb, 256, 0, st>>>(s->P, s->V, s->cell_of, s->start, e.total, s->arrival,
                                         s->order, s->SP, s->SV);
-        const bool lanes = n <= s->warp_max && n <= kSphLanesMax;
-        if (lanes && n <= kSph16Max) {
-            launch_density<16>(s, st);
-            launch_force<16>(s, out, st);
-        } else if (lanes) {
-            launch_density<8>(s, st);
-            launch_force<8>(s, out, st);
-        } else {
-            if (n <= kSphDensity8Max) launch_density<8>(s, st);
-            else launch_density<1>(s, st);
-            launch_force<1>(s, out, st);
-        }
+        const bool fastest = s->warp_max < 0;
+        const bool lanes_f = n <= (fastest ? kSphLanesMax : s->warp_max);
+        const bool lanes_d = n <= (fastest ? kSphDensity8Max : s->warp_max);
+        if (!lanes_d) launch_density<1>(s, st);
+        else if (n <= kSph16Max) launch_density<16>(s, st);
+        else launch_density<8>(s, st);
+        if (!lanes_f) launch_force<1>(s, out, st);
+        else if (n <= kSph16Max) launch_force<16>(s, out, st);
+        else launch_force<8>(s, out, st);
     }
 }
 
@@ -1163,13 +1159,16 @@ int mpm_sph_set_graph(mpm_sph* s, int enable) {
 
 int mpm_sph_set_warp_per_particle(mpm_sph* s, int max_particles) {
     if (!s || max_particles < -1) return fail(MPM_E_INVALID, "bad arguments");
-    const int v = max_particles == -1 ? kSphWarpMaxDefault : max_particles;
+    const int v = max_particles == kSphWarpMaxDefault ? -1 : max_particles;
     if (v != s->warp_max) drop_graphs(s);  // the captured frames hold the launches
     s->warp_max = v;
     return MPM_OK;
 }
 
-int mpm_sph_get_warp_per_particle(const mpm_sph* s) { return s ? s->warp_max : MPM_E_INVALID; }
+int mpm_sph_get_warp_per_particle(const mpm_sph* s) {
+    if (!s) return MPM_E_INVALID;
+    return s->warp_max < 0 ? kSphWarpMaxDefault : s->warp_max;
+}
 
 int mpm_sph_num_particles(const mpm_sph* s) { return s ? s->n : 0; }
 int64_t mpm_sph_grid_count(const mpm_sph* s) { return s ? s->e.total : 0; }

@@ -60,9 +60,10 @@ class SPHSimulator:
 
     @property
     def warpPerParticle(self) -> int:
-        """Particle counts up to this may run the forces with several lanes of
-        a warp per particle, and do where that is the faster way (default
-        32768; 0: never; -1 to set: the default).  Results are the same."""
+        """Particle counts up to this run density and forces with several lanes
+        of a warp per particle, others with a thread (0: always a thread; -1 or
+        32768, the default: the faster at each particle count).  Results are
+        the same."""
         return _check(self._lib.mpm_sph_get_warp_per_particle(self._handle), "warpPerParticle")
 
     @warpPerParticle.setter
