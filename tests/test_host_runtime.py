@@ -102,3 +102,25 @@ def test_sph_lanes_per_particle(fake, pkg, n, warp_max, density, force):
     sim.warpPerParticle = -1
     assert sim.warpPerParticle == 32768
     sim.close()
+
+
+@pytest.mark.parametrize("box,chunk_sums,one_launch", [
+    ((32, 32, 32), False, True),     # 514 bins
+    ((124, 44, 48), False, True),    # 4,094
+    ((64, 64, 64), False, False),    # 4,098
+    ((80, 80, 80), False, False),    # 8,002: 32 chunks
+    ((84, 80, 80), True, False),     # 8,402: 33 chunks
+    ((128, 128, 128), True, False),  # 32,770: 129 chunks
+])
+def test_scan_launches(fake, pkg, box, chunk_sums, one_launch):
+    """The counting sort's launches by the scene's bins, as measured."""
+    sim = pkg.MLSMPMSimulator(None, None, maxParticles=100, maxGrid=box)
+    sim.setGraph(False)
+    sim.upload(np.full((100, 20), 5.0, np.float32), [float(b) for b in box])
+    sim.execute()
+    fake.fake_reset(-1)
+    sim.execute()
+    ran = fake.fake_launched().decode()
+    assert ("k_chunk_sums" in ran) == chunk_sums
+    assert ("k_scan_scatter" in ran) == one_launch
+    sim.close()

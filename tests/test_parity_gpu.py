@@ -600,3 +600,22 @@ def test_constants_that_change_between_calls(cuda, pkg, oracle_mod):
         ref.execute(2, NTHREADS)
     assert_state_equal(sim, ref, "after 24 frames")
     sim.close()
+
+
+@pytest.mark.parametrize("box", [(80, 80, 80), (84, 80, 80)])
+def test_chunk_sums_edge(cuda, pkg, oracle_mod, box):
+    """Either side of the most scan chunks without chunk sums (8,002 bins are
+    32 chunks, 8,402 are 33), particles over the whole box."""
+    rng = np.random.default_rng(box[0])
+    recs = np.zeros((5000, 20), np.float32)
+    recs[:, 0:3] = 2.0 + rng.random((5000, 3)) * (np.array(box) - 4.5)
+    recs[:1500, 0:3] = np.array(box) - 6.0 + rng.random((1500, 3))
+    recs[:, 4:7] = rng.normal(0.0, 0.5, (5000, 3))
+    sim = make_sim(pkg, "sorted", max_particles=5000, max_grid=box)
+    sim.upload(recs, [float(b) for b in box])
+    ref = oracle_mod.OracleSim(sim.downloadParticles(), [float(b) for b in box])
+    for _ in range(2):
+        sim.execute()
+        ref.execute(2, NTHREADS)
+    assert_state_equal(sim, ref, f"box {box}")
+    sim.close()

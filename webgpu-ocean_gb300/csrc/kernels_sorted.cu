@@ -102,9 +102,13 @@ constexpr int kPairDefaultRequest = INT_MAX;  // sorted_set_pair_max: restore th
 // 5.9 -> 3.6 us, at a million 8.6 -> 4.4 us and 3.2 us for the chunk sums).
 constexpr int kScanThreads = 256;
 // With more bin chunks (of kScanThreads bins) than this, k_chunk_sums sums
-// each chunk once before k_scan (a million particles, 133 chunks: frame 376 us
-// with the chunk sums, 393 us with every CTA adding up the bins before its own).
-constexpr int kChunkedScanMin = 128;
+// each chunk once before k_scan, which costs a launch; with fewer, every CTA
+// adds up the bins before its own.  Frames of 30,000 / 200,000 particles in us,
+// without and with the chunk sums: 17 chunks 66.6, 68.0 / 141.1, 141.6, 26 chunks
+// 67.8, 68.1 / 140.4, 140.5, 32 chunks 69.9, 69.0 / 136.5, 136.4, 55 chunks 70.1,
+// 67.6 / 136.6, 133.3, 86 chunks 86.3, 79.7 / 139.7, 133.1, 106 chunks 88.3, 80.1
+// / 141.1, 132.1, 129 chunks 90.6, 80.1 / 146.6, 136.0.
+constexpr int kChunkedScanMin = 32;
 // Most bins of a scene whose scan and scatter are one launch (see
 // k_scan_scatter), and the particles of a thread of its scatter.
 constexpr int kFusedBins = 4096;
@@ -1088,7 +1092,7 @@ __global__ void __launch_bounds__(kTask) k_bin(Particles P, Scene one, Dev d, in
 // kScanThreads bins from c*kScanThreads; it finds its starting offsets by
 // reducing all earlier counts itself, from L2, or k_chunk_sums' sums where
 // there are many, so no CTA waits on another.  The counts are zeroed by
-// k_scatter, which runs next.
+// k_scatter, which runs next, or by k_update where the two are one launch.
 
 constexpr int kScanWarps = kScanThreads / 32;
 
@@ -1324,9 +1328,11 @@ __global__ void k_scatter(Dev d, int n, int nbins) {
 // first slots of all bins itself, in shared memory, for kFusedScatter particles a
 // thread, so that none waits for another.  The counts stay: k_update zeroes them.
 // A launch fewer a substep; frames with two launches and with one: 3,000
-// particles (214 bins) 51.3 / 49.1 us, 70,000 with their image (1,202 bins) 226.8 /
-// 223.8, 200,000 (3,382 bins) 163.4 / 158.2.  Above, the bins each CTA
-// adds up again weigh more, and the frame is long against a launch.
+// particles (242 bins) 51.3 / 49.1 us, 70,000 with their image (1,282 bins) 226.8 /
+// 223.8, 200,000 (3,382 bins) 163.4 / 158.2, 200,000 (3,842 bins) 140.2 / 137.2.
+// The more bins, the more each CTA adds up again: with the limit raised
+// 200,000 particles gain less (4,098 bins 141.1 / 139.4, 6,482 bins 140.2 /
+// 137.7) and lose at 8,002 bins (136.5 / 139.4).
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_scatter(Dev d, Geo one_g, int n, int nbins, int chunks) {
     __shared__ uint32_t s_scan[3 * kScanWarps];
@@ -1431,7 +1437,7 @@ struct SortedEngine {
     int blocks_p2g2() const { return std::min(blocks_p2g2_v[variant()], most_tasks()); }
     int blocks_g2p() const { return std::min(blocks_g2p_v[variant()], most_tasks()); }
     // No more CTAs than there can be tasks: a task per bin and one more for
-    // every task_cap particles.  3,000 particles in 212 bins: 259 CTAs instead
+    // every task_cap particles.  3,000 particles in 242 bins: 289 CTAs instead
     // of 608 (frame 53.4 -> 51.0 us).
     long long particles = 0;
     int most_tasks() const {
