@@ -3,11 +3,12 @@
 // the real one.  Device memory is host memory, copies and memsets are done at
 // once, kernels are noted and not run.
 //
-// Besides, it keeps the one rule of order that a caller on a stream of its own
+// Besides, it keeps the rules of order that a caller on a stream of its own
 // depends on: copies from pageable memory and memsets on the null stream may
-// return before they are done, and a non-blocking stream does not wait for them.
-// fake_unordered() counts the kernels and graphs that were launched on another
-// stream with such work outstanding.
+// return before they are done, and neither they nor the work on a non-blocking
+// stream wait for one another.  fake_unordered() counts the kernels and graphs
+// launched on another stream with such work outstanding, and the copies and
+// memsets on the null stream with such kernels or graphs outstanding.
 #include <cuda_runtime_api.h>
 
 #include <cstdlib>
@@ -23,6 +24,7 @@ size_t g_used = 0;
 std::map<void*, size_t> g_size;
 cudaError_t g_error = cudaSuccess;
 bool g_pending = false;      // null-stream work that nothing has waited for
+bool g_busy = false;         // kernels or graphs on another stream, likewise
 int g_unordered = 0;
 std::map<const void*, std::string> g_name;  // mangled, by host stub
 std::string g_launched;                     // names, a line each
@@ -43,10 +45,20 @@ cudaError_t issued(cudaStream_t st) {
     return cudaSuccess;
 }
 
+cudaError_t copied(cudaStream_t st) {
+    if (!st && g_busy) ++g_unordered;
+    return issued(st);
+}
+
+cudaError_t ran(cudaStream_t st) {
+    if (st && g_pending) ++g_unordered;
+    if (st) g_busy = true;
+    return issued(st);
+}
+
 cudaError_t launched(const void* f, cudaStream_t st) {
     g_launched += g_name[f] + "\n";
-    if (st && g_pending && !g_capturing.count(st)) ++g_unordered;
-    return issued(st);
+    return g_capturing.count(st) ? cudaSuccess : ran(st);
 }
 
 template <class T>
@@ -68,7 +80,7 @@ extern "C" {
 void fake_reset(size_t room) {
     g_room = room;
     g_error = cudaSuccess;
-    g_pending = false;
+    g_pending = g_busy = false;
     g_unordered = 0;
     g_launched.clear();
 }
@@ -126,25 +138,25 @@ cudaError_t cudaFreeAsync(void* p, cudaStream_t) { return cudaFree(p); }
 
 cudaError_t cudaMemcpy(void* to, const void* from, size_t bytes, cudaMemcpyKind kind) {
     std::memmove(to, from, bytes);
+    copied(nullptr);
     if (kind == cudaMemcpyDeviceToHost) g_pending = false;  // returns when it is done
-    else g_pending = true;
     return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void* to, const void* from, size_t bytes, cudaMemcpyKind, cudaStream_t st) {
     std::memmove(to, from, bytes);
-    return issued(st);
+    return copied(st);
 }
 cudaError_t cudaMemset(void* p, int v, size_t bytes) {
     std::memset(p, v, bytes);
-    return issued(nullptr);
+    return copied(nullptr);
 }
 cudaError_t cudaMemsetAsync(void* p, int v, size_t bytes, cudaStream_t st) {
     std::memset(p, v, bytes);
-    return issued(st);
+    return copied(st);
 }
-cudaError_t cudaDeviceSynchronize() { g_pending = false; return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize() { g_pending = g_busy = false; return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t st) {
-    if (!st) g_pending = false;
+    (st ? g_busy : g_pending) = false;
     return cudaSuccess;
 }
 
@@ -162,10 +174,7 @@ cudaError_t cudaStreamEndCapture(cudaStream_t s, cudaGraph_t* g) {
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long) { return made(e); }
 cudaError_t cudaGraphDestroy(cudaGraph_t g) { return gone(g); }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t e) { return gone(e); }
-cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t st) {
-    if (st && g_pending) ++g_unordered;
-    return issued(st);
-}
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t st) { return ran(st); }
 cudaError_t cudaEventCreate(cudaEvent_t* e) { return made(e); }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return made(e); }
 cudaError_t cudaEventDestroy(cudaEvent_t e) { return gone(e); }

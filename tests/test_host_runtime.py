@@ -124,3 +124,39 @@ def test_scan_launches(fake, pkg, box, chunk_sums, one_launch):
     assert ("k_chunk_sums" in ran) == chunk_sums
     assert ("k_scan_scatter" in ran) == one_launch
     sim.close()
+
+
+def _scenes(pkg):
+    return [pkg.scene_desc(40, [16.0, 12.0, 20.0]), pkg.scene_desc(24, [14.0, 14.0, 14.0])]
+
+
+def _use_simulator(pkg):
+    sim = pkg.MLSMPMSimulator(None, None, maxParticles=64, maxGrid=(16, 16, 16))
+    recs = np.full((64, 20), 5.0, np.float32)
+    for graph in (True, False):
+        sim.setGraph(graph)
+        sim.upload(recs, [16.0, 16.0, 16.0])
+        sim.execute(SIDE_STREAM)
+        sim.changeBoxSize([16.0, 16.0, 15.0])
+        sim.execute(SIDE_STREAM)
+    sim.close()
+
+
+def _use_batch(pkg):
+    recs = np.full((64, 20), 5.0, np.float32)
+    batch = pkg.MLSMPMBatch(_scenes(pkg), recs)
+    batch.step(2, SIDE_STREAM)
+    batch.setScene(0, pkg.scene_desc(40, [16.0, 12.0, 20.0], stiffness=2.0))
+    batch.step(2, SIDE_STREAM)
+    batch.upload(recs)
+    batch.step(2, SIDE_STREAM)
+    batch.close()
+
+
+@pytest.mark.parametrize("use", [_use_simulator, _use_batch])
+def test_streams_and_uploads_in_order(fake, pkg, use):
+    """Work on the caller's own stream finds what was uploaded before it, and
+    an upload waits for the work in flight."""
+    use(pkg)
+    assert fake.fake_launched()
+    assert fake.fake_unordered() == 0

@@ -591,9 +591,8 @@ int mpm_adjoint_set_tape(mpm_adjoint* a, int tape) {
 
 int mpm_adjoint_set_scene(mpm_adjoint* a, int scene, const mpm_scene_desc* desc) {
     if (!a) return fail(MPM_E_INVALID, "null adjoint handle");
-    if (int rc = mpm_batch_set_scene(a->b, scene, desc)) return rc;
+    if (int rc = mpm_batch_set_scene(a->b, scene, desc)) return rc;  // waits for the device
     DeviceGuard g(a->b->device);
-    MPM_CUDA(cudaDeviceSynchronize());
     a->T = -1;
     return upload_adj_scenes(a);
 }

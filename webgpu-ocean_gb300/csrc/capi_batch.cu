@@ -181,10 +181,13 @@ int mpm_batch_set_scene(mpm_batch* b, int scene, const mpm_scene_desc* desc) {
     SimConsts k;
     if (int rc = scene_consts(*desc, k)) return rc;
     DeviceGuard g(b->device);
+    // steps in flight on any stream keep their constants, the next ones have the new
+    MPM_CUDA(cudaDeviceSynchronize());
     if (sorted_set_scene_consts(b->sorted, scene, k, nullptr) != 0)
         return fail(MPM_E_INVALID, std::string("batch: ") + sorted_error());
     b->desc[(size_t)scene] = *desc;
     b->consts[(size_t)scene] = k;
+    MPM_CUDA(cudaStreamSynchronize(nullptr));
     return MPM_OK;
 }
 
