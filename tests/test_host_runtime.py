@@ -153,7 +153,23 @@ def _use_batch(pkg):
     batch.close()
 
 
-@pytest.mark.parametrize("use", [_use_simulator, _use_batch])
+def _use_adjoint(pkg, tape):
+    recs = np.full((64, 20), 5.0, np.float32)
+    adj = pkg.MLSMPMAdjoint(_scenes(pkg), 4, 2, tape=tape)
+    for _ in range(2):
+        adj.forward(recs, 4, SIDE_STREAM)
+        adj.setObservations({4: np.zeros((64, 3), np.float32)})
+        adj.observationLoss(SIDE_STREAM)
+        adj.backwardObserved(SIDE_STREAM)
+        adj.setScene(0, pkg.scene_desc(40, [16.0, 12.0, 20.0], stiffness=2.0))
+    adj.forward(recs, 4, SIDE_STREAM)
+    adj.backward({4: recs}, SIDE_STREAM)
+    adj.close()
+
+
+@pytest.mark.parametrize("use", [
+    _use_simulator, _use_batch, lambda pkg: _use_adjoint(pkg, "fp64"), lambda pkg: _use_adjoint(pkg, "fixed"),
+], ids=["simulator", "batch", "adjoint fp64", "adjoint fixed"])
 def test_streams_and_uploads_in_order(fake, pkg, use):
     """Work on the caller's own stream finds what was uploaded before it, and
     an upload waits for the work in flight."""

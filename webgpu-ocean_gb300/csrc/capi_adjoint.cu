@@ -609,6 +609,7 @@ int mpm_forward_ckpt(mpm_adjoint* a, const float* init, int substeps, void* stre
     a->T = -1;
     a->obs_seeded = false;
     MPM_CUDA(cudaStreamSynchronize(st));
+    MPM_CUDA(cudaStreamSynchronize(nullptr));  // the scenes' copies, which nothing has waited for
     // The last checkpoint segment is the first one the backward needs: its
     // states and updated grids are recorded here, as the backward's
     // recompute would record them, so that it is not recomputed.
@@ -758,6 +759,7 @@ int mpm_adjoint_set_observations(mpm_adjoint* a, int count, const int* substeps,
     }
     MPM_CUDA(cudaMemcpy(a->obs_scale, scale.data(), sizeof(float) * (size_t)S,
                         cudaMemcpyHostToDevice));
+    MPM_CUDA(cudaStreamSynchronize(nullptr));  // a copy from pageable memory may outlast its call
     return MPM_OK;
 }
 
