@@ -167,9 +167,20 @@ def _use_adjoint(pkg, tape):
     adj.close()
 
 
+def _use_renderer(pkg):
+    posvel = np.zeros((8, 8), np.float32)
+    u = pkg.camera_uniforms(64, 48, 40.0, [10.0, 4.0, 12.0], 0.8, 1.2)
+    r = pkg.FluidRenderer(64, 48, 0.6, 0.8)
+    for spheres in (True, False):
+        r.execute(posvel.ctypes.data, 8, u, SIDE_STREAM, sphereRenderFl=spheres)
+    r.setEnvmap(np.ones((6, 4, 4, 4), np.float32))
+    r.execute(posvel.ctypes.data, 8, u, SIDE_STREAM)
+    r.close()
+
+
 @pytest.mark.parametrize("use", [
     _use_simulator, _use_batch, lambda pkg: _use_adjoint(pkg, "fp64"), lambda pkg: _use_adjoint(pkg, "fixed"),
-], ids=["simulator", "batch", "adjoint fp64", "adjoint fixed"])
+    _use_renderer], ids=["simulator", "batch", "adjoint fp64", "adjoint fixed", "renderer"])
 def test_streams_and_uploads_in_order(fake, pkg, use):
     """Work on the caller's own stream finds what was uploaded before it, and
     an upload waits for the work in flight."""

@@ -1224,6 +1224,9 @@ int upload_env(mpm_renderer* r, int size, const float* rgba) {
     cudaError_t err = cudaMalloc(&e, sizeof(float4) * 6 * (size_t)size * size);
     if (err == cudaSuccess)
         err = cudaMemcpy(e, rgba, sizeof(float4) * 6 * (size_t)size * size, cudaMemcpyHostToDevice);
+    // the copy from pageable memory may outlast its call, and an image on a
+    // non-blocking stream would not wait for it
+    if (err == cudaSuccess) err = cudaStreamSynchronize(nullptr);
     if (err != cudaSuccess) {
         cudaFree(e);
         return cuda_fail(err, "envmap");
