@@ -249,9 +249,11 @@ int mpm_get_bin_pairing(const mpm_sim* sim);
  * 256, 512, 2^30}, each task-kernel block size in {128, 256, 512}, each task
  * size in {128, 256, 512, 1024} and each lane-table threshold in {32, 128,
  * 512, off} from the current state (each combination once untimed first, so
- * its CUDA graphs are captured outside the timing), then the fastest twelve
- * over five times as many, keeps the fastest of those and restores the state (particles, posvel, counters and grid are as before
- * the call).  Writes the task size to *chosen_task_size when non-null (the
+ * its CUDA graphs are captured outside the timing).  Then, over five times as
+ * many, it times the fastest twelve (each with its best lane-table threshold)
+ * and the other thresholds of the fastest of those, keeps the fastest and
+ * restores the state (particles, posvel, counters and grid are as before the
+ * call).  Writes the task size to *chosen_task_size when non-null (the
  * others: mpm_get_bin_pairing, mpm_get_task_threads,
  * mpm_get_lane_table_min).  Synchronizes. */
 int mpm_autotune(mpm_sim* sim, int substeps, int* chosen_task_size);

@@ -29,6 +29,9 @@ int g_unordered = 0;
 std::map<const void*, std::string> g_name;  // mangled, by host stub
 std::string g_launched;                     // names, a line each
 std::set<cudaStream_t> g_capturing;
+float (*g_elapsed)(int) = nullptr;  // time of that many graphs in a row
+int g_graphs = 0;                   // launched since the last event
+int g_between = 0;                  // between the last two events
 struct Config {
     dim3 grid, block;
     size_t smem;
@@ -83,7 +86,9 @@ void fake_reset(size_t room) {
     g_pending = g_busy = false;
     g_unordered = 0;
     g_launched.clear();
+    g_elapsed = nullptr;
 }
+void fake_elapsed(float (*ms)(int)) { g_elapsed = ms; }
 int fake_unordered() { return g_unordered; }
 size_t fake_used() { return g_used; }
 const char* fake_launched() { return g_launched.c_str(); }
@@ -174,14 +179,21 @@ cudaError_t cudaStreamEndCapture(cudaStream_t s, cudaGraph_t* g) {
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long) { return made(e); }
 cudaError_t cudaGraphDestroy(cudaGraph_t g) { return gone(g); }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t e) { return gone(e); }
-cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t st) { return ran(st); }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t st) {
+    ++g_graphs;
+    return ran(st);
+}
 cudaError_t cudaEventCreate(cudaEvent_t* e) { return made(e); }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return made(e); }
 cudaError_t cudaEventDestroy(cudaEvent_t e) { return gone(e); }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) {
+    g_between = g_graphs;
+    g_graphs = 0;
+    return cudaSuccess;
+}
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) {
-    *ms = 1.0f;
+    *ms = g_elapsed ? g_elapsed(g_between) : 1.0f;
     return cudaSuccess;
 }
 

@@ -187,3 +187,25 @@ def test_streams_and_uploads_in_order(fake, pkg, use):
     use(pkg)
     assert fake.fake_launched()
     assert fake.fake_unordered() == 0
+
+
+def test_autotune_chooses_by_the_longer_timing(fake, pkg):
+    """What is the fastest over one window of substeps need not be over five:
+    every part of the choice is by the longer timing."""
+    sim = pkg.MLSMPMSimulator(None, None, maxParticles=64, maxGrid=(16, 16, 16))
+    sim.upload(np.full((64, 20), 5.0, np.float32), [16.0, 16.0, 16.0])
+    timed = []
+
+    @ctypes.CFUNCTYPE(ctypes.c_float, ctypes.c_int)
+    def elapsed(windows):
+        t = sim.tuning()
+        ms = 10.0 + (t["task_threads"] != 256) + (t["task_size"] != 512) + (t["bin_pairing"] != 0)
+        short, long = t["lane_table_min"] == 32, t["lane_table_min"] == 512
+        timed.append(windows)
+        return windows * ms - (0.5 if windows == 1 and short else 0.0) - (2.5 if windows > 1 and long else 0.0)
+
+    fake.fake_elapsed(elapsed)
+    assert sim.autotune(8) == 512
+    assert sim.tuning() == {"bin_pairing": 0, "task_threads": 256, "task_size": 512, "lane_table_min": 512}
+    assert set(timed) == {1, 5}
+    sim.close()

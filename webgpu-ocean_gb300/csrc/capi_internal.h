@@ -67,8 +67,9 @@ int scene_consts(const mpm_scene_desc& d, SimConsts& k);
 
 // Times `substeps` sorted-engine substeps for each combination of z-pair
 // threshold, task-kernel block size, task size and lane-table threshold from
-// the same saved state, the fastest of them once more over five times as many,
-// and keeps the fastest of those.  Each candidate first runs once untimed, so that
+// the same saved state; then, over five times as many, the fastest of them and
+// the other lane-table thresholds of the fastest of those, and keeps the fastest
+// by that timing.  Each candidate first runs once untimed, so that
 // the CUDA graphs the timed run replays are captured outside it.  The state
 // after the call is the state before it (particles, posvel, counters, grid).
 template <class StepFn>
@@ -168,17 +169,15 @@ int tune_engine(SortedEngine* e, ParticleStore& ps, int n, float4* posvel,
     }
     std::stable_sort(found.begin(), found.end(), faster);
     if (found.size() > kFinalists) found.resize(kFinalists);
-    int best = 0, best_lane = 0, best_threads = 0, best_pair = 0;
-    double best_ms = 0.0;
-    for (Choice& c : found) {
-        if (err != cudaSuccess) break;
-        if (!time_choice(c, kWindows) || (best && c.ms >= best_ms)) continue;
-        best = c.cap;
-        best_lane = c.lane;
-        best_threads = c.threads;
-        best_pair = c.pair;
-        best_ms = c.ms;
-    }
+    Choice best{0, 0, 0, 0, 0.f};
+    auto keep_faster = [&](Choice c) {
+        if (err == cudaSuccess && time_choice(c, kWindows) && (!best.cap || faster(c, best))) best = c;
+    };
+    for (const Choice& c : found) keep_faster(c);
+    // the lane-table threshold too by the longer timing
+    const Choice first = best;
+    for (int lane : kLanes)
+        if (first.cap && lane != first.lane) keep_faster({first.pair, first.threads, first.cap, lane, 0.f});
     if (err == cudaSuccess) err = restore();
     if (err == cudaSuccess)
         err = cudaMemcpyAsync(posvel, pv, sizeof(float4) * 2 * (size_t)n, cudaMemcpyDeviceToDevice, st);
@@ -186,16 +185,16 @@ int tune_engine(SortedEngine* e, ParticleStore& ps, int n, float4* posvel,
     if (err == cudaSuccess) err = cudaStreamSynchronize(st);
     cleanup();
     if (err != cudaSuccess) return cuda_fail(err, "autotune");
-    if (best) {
-        sorted_set_pair_max(e, best_pair);
-        sorted_set_threads(e, best_threads);
-        sorted_set_task_cap(e, best);
-        sorted_set_lane_table_min(e, best_lane);
+    if (best.cap) {
+        sorted_set_pair_max(e, best.pair);
+        sorted_set_threads(e, best.threads);
+        sorted_set_task_cap(e, best.cap);
+        sorted_set_lane_table_min(e, best.lane);
     }
-    if (chosen) *chosen = best;
-    if (chosen_lane) *chosen_lane = best_lane;
-    if (chosen_threads) *chosen_threads = best_threads;
-    if (ms_out) *ms_out = best_ms / kWindows;
+    if (chosen) *chosen = best.cap;
+    if (chosen_lane) *chosen_lane = best.lane;
+    if (chosen_threads) *chosen_threads = best.threads;
+    if (ms_out) *ms_out = (double)best.ms / kWindows;
     return MPM_OK;
 }
 
