@@ -292,7 +292,9 @@ int mpm_batch_step(mpm_batch* batch, int substeps, void* stream);
  * captured graphs are kept (synchronizes). */
 int mpm_batch_upload(mpm_batch* batch, const float* aos80);
 /* Replaces scene s's constants (box sizes and num_particles must stay) for the
- * steps that follow (synchronizes). */
+ * steps that follow on any stream, and for later replays of captured ones;
+ * steps in flight keep theirs (waits for them).  Synchronize between this and
+ * a capture of steps. */
 int mpm_batch_set_scene(mpm_batch* batch, int scene, const mpm_scene_desc* desc);
 int mpm_batch_set_graph(mpm_batch* batch, int enable); /* default 1 */
 int mpm_batch_set_task_size(mpm_batch* batch, int task_size); /* see mpm_set_task_size */

@@ -172,6 +172,10 @@ cudaError_t cudaStreamBeginCapture(cudaStream_t s, cudaStreamCaptureMode) {
     g_capturing.insert(s);
     return cudaSuccess;
 }
+cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus* status) {
+    *status = g_capturing.count(s) ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+    return cudaSuccess;
+}
 cudaError_t cudaStreamEndCapture(cudaStream_t s, cudaGraph_t* g) {
     g_capturing.erase(s);
     return made(g);
@@ -181,7 +185,7 @@ cudaError_t cudaGraphDestroy(cudaGraph_t g) { return gone(g); }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t e) { return gone(e); }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t st) {
     ++g_graphs;
-    return ran(st);
+    return g_capturing.count(st) ? cudaSuccess : ran(st);
 }
 cudaError_t cudaEventCreate(cudaEvent_t* e) { return made(e); }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return made(e); }

@@ -150,6 +150,15 @@ def _use_batch(pkg):
     batch.step(2, SIDE_STREAM)
     batch.upload(recs)
     batch.step(2, SIDE_STREAM)
+    rt = pkg._lib.load()
+    stream, graph = ctypes.c_void_p(SIDE_STREAM), ctypes.c_void_p()
+    rt.cudaStreamBeginCapture(stream, 0)
+    batch.step(2, SIDE_STREAM)
+    rt.cudaStreamEndCapture(stream, ctypes.byref(graph))
+    for stiffness in (3.0, 4.0):
+        rt.cudaGraphLaunch(graph, stream)
+        batch.setScene(1, pkg.scene_desc(24, [14.0, 14.0, 14.0], stiffness=stiffness))
+    rt.cudaGraphLaunch(graph, stream)
     batch.close()
 
 

@@ -54,6 +54,7 @@ struct mpm_adjoint {
     // substeps) and replayed while they stay the same.
     cudaGraphExec_t bgraph = nullptr;
     int bg_T = -1, bg_every = 0, bg_tape = -1, bg_cur = 0;
+    bool scenes_set = false;         // scenes have constants that scenes_d does not
     bool last_taped = false;         // the forward recorded its last segment's tape
     bool bg_last_taped = false;
     bool bg_fast_dec = true;         // the kernels it was captured with (all_fast_dec)
@@ -591,10 +592,10 @@ int mpm_adjoint_set_tape(mpm_adjoint* a, int tape) {
 
 int mpm_adjoint_set_scene(mpm_adjoint* a, int scene, const mpm_scene_desc* desc) {
     if (!a) return fail(MPM_E_INVALID, "null adjoint handle");
-    if (int rc = mpm_batch_set_scene(a->b, scene, desc)) return rc;  // waits for the device
-    DeviceGuard g(a->b->device);
+    if (int rc = mpm_batch_set_scene(a->b, scene, desc)) return rc;
     a->T = -1;
-    return upload_adj_scenes(a);
+    a->scenes_set = true;  // copied by the next forward, which everything else needs first
+    return MPM_OK;
 }
 
 int mpm_forward_ckpt(mpm_adjoint* a, const float* init, int substeps, void* stream) {
@@ -609,6 +610,10 @@ int mpm_forward_ckpt(mpm_adjoint* a, const float* init, int substeps, void* stre
     a->T = -1;
     a->obs_seeded = false;
     MPM_CUDA(cudaStreamSynchronize(st));
+    b->in_flight = true;  // for the next scene that is set
+    if (a->scenes_set)
+        if (int rc = upload_adj_scenes(a)) return rc;
+    a->scenes_set = false;
     MPM_CUDA(cudaStreamSynchronize(nullptr));  // the scenes' copies, which nothing has waited for
     // The last checkpoint segment is the first one the backward needs: its
     // states and updated grids are recorded here, as the backward's

@@ -45,6 +45,22 @@ int scene_consts(const mpm_scene_desc& d, SimConsts& k) {
     return MPM_OK;
 }
 
+// Before steps on `st`, which read the scenes' constants.  The null stream is in
+// order by itself, and nothing can wait in a capture.
+cudaError_t after_scene_copies(mpm_batch* b, cudaStream_t st) {
+    if (!st) return cudaSuccess;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (const cudaError_t e = cudaStreamIsCapturing(st, &capture)) return e;
+    if (capture != cudaStreamCaptureStatusNone) {
+        b->captured = true;
+        return cudaSuccess;
+    }
+    b->in_flight = true;
+    if (!b->copies) return cudaSuccess;
+    b->copies = false;
+    return cudaStreamSynchronize(nullptr);
+}
+
 }  // namespace mpm
 
 namespace {
@@ -148,6 +164,7 @@ int mpm_batch_step(mpm_batch* b, int substeps, void* stream) {
     DeviceGuard g(b->device);
     if (!g.ok) return fail(MPM_E_CUDA, "cannot select the batch's device");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    MPM_CUDA(after_scene_copies(b, st));
     if (sorted_step(b->sorted, &b->ps, b->posvel, b->counters, b->consts[0], substeps, st, &b->prof,
                     b->graph) != 0)
         return fail(MPM_E_CUDA, std::string("batch: ") + sorted_error());
@@ -181,13 +198,15 @@ int mpm_batch_set_scene(mpm_batch* b, int scene, const mpm_scene_desc* desc) {
     SimConsts k;
     if (int rc = scene_consts(*desc, k)) return rc;
     DeviceGuard g(b->device);
-    // steps in flight on any stream keep their constants, the next ones have the new
-    MPM_CUDA(cudaDeviceSynchronize());
+    // steps in flight keep their constants
+    if (b->in_flight || b->captured) MPM_CUDA(cudaDeviceSynchronize());
+    b->in_flight = false;
+    b->copies = true;
     if (sorted_set_scene_consts(b->sorted, scene, k, nullptr) != 0)
         return fail(MPM_E_INVALID, std::string("batch: ") + sorted_error());
     b->desc[(size_t)scene] = *desc;
     b->consts[(size_t)scene] = k;
-    MPM_CUDA(cudaStreamSynchronize(nullptr));
+    if (b->captured) MPM_CUDA(cudaStreamSynchronize(nullptr));
     return MPM_OK;
 }
 

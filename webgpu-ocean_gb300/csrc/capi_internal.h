@@ -212,9 +212,14 @@ struct mpm_batch {
     mpm::SortedEngine* sorted = nullptr;
     bool graph = true;
     bool stepped = false;
+    // order between scenes' new constants, copied on the null stream, and work on
+    // other streams: work that a copy has to wait for, copies that work has to
+    // wait for, and whether steps were captured (their replays are not seen here)
+    bool in_flight = false, copies = false, captured = false;
     mpm::LaunchProfiler prof;
 };
 
 namespace mpm {
 int check_batch(const mpm_batch* b);  // capi_batch.cu
+cudaError_t after_scene_copies(mpm_batch* b, cudaStream_t st);
 }  // namespace mpm
