@@ -310,12 +310,13 @@ def run_reference(args) -> None:
 
 
 # DRAM bytes (read + write) per launch of the dominant kernel, from one ncu
-# capture of `bench.py --quick` on this workload: its posvel-writing variant
-# (profiles/k_g2p_p2g1_1M_128.md).
-MEASURED_TRAFFIC_PER_LAUNCH = {"sorted_g2p_p2g_1": 93.59e6}
-# ncu smsp__inst_executed.sum of one launch at the early dam-break state
-# (profiles/k_g2p_p2g1_1M_128.md): the instruction-issue roofline.
-MEASURED_WARP_INSTRUCTIONS_PER_LAUNCH = {"sorted_g2p_p2g_1": 70.22e6}
+# capture of `bench.py --quick --no-autotune` on this workload: its
+# posvel-writing variant, at the early dam-break state and the engine's default
+# tuning (256 threads, tasks of 1024).  The timed run is autotuned and may split
+# its tasks otherwise.
+MEASURED_TRAFFIC_PER_LAUNCH = {"sorted_g2p_p2g_1": 93.69e6}
+# smsp__inst_executed.sum of the same launch: the instruction-issue roofline.
+MEASURED_WARP_INSTRUCTIONS_PER_LAUNCH = {"sorted_g2p_p2g_1": 70.24e6}
 
 
 def algorithmic_bytes(kernel: str, n: int, cells: int) -> float | None:
@@ -997,8 +998,8 @@ def run_ours(args) -> None:
                 "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "peak_source": peaks["source"],
                 "traffic": MEASURED_TRAFFIC_PER_LAUNCH.get(top_name),
-                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum, "
-                                  "profiles/k_g2p_p2g1_1M_128.md",
+                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one "
+                                  "early-state launch at the default tuning",
                 "algorithmic_bytes_per_launch": abytes,
                 "mean_launch_us": avg_s * 1e6, "cells_touched": cells,
                 "kernel_share": top_ms / step_kernel_ms if step_kernel_ms else None}
@@ -1014,8 +1015,8 @@ def run_ours(args) -> None:
         issue = {"kernel": top_name, "achieved": got / 1e12, "peak": peak_issue / 1e12,
                  "unit": "T warp-instructions/s", "frac": got / peak_issue,
                  "warp_instructions_per_launch": instr,
-                 "source": "ncu smsp__inst_executed.sum of one early-state launch, "
-                           "profiles/k_g2p_p2g1_1M_128.md; peak = 4 x SMs x median SM clock"}
+                 "source": "ncu smsp__inst_executed.sum of one early-state launch at the default "
+                           "tuning, over this run's mean duration; peak = 4 x SMs x median SM clock"}
     kernels = {k: {"launches": v[0], "mean_us": 1e3 * v[2] / v[1] if v[1] else None,
                    "share": v[2] / step_kernel_ms if step_kernel_ms else None}
                for k, v in stats.items()}

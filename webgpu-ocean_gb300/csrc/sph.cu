@@ -292,9 +292,10 @@ __device__ __forceinline__ float dist2(const float4& a, const float4& b) {
 // Markstein's final one, which rounds correctly because the remainder
 // fma(-b, q, a) is exact (P. Markstein, IBM J. Res. Dev. 34, 1990).  Five
 // operations instead of a division.  Holds for quotients in [kQuotMin,
-// kQuotMax] when b lies in [2^-20, 2^40]: no intermediate leaves the normal
-// range.  rcp_for_quotients(b) is NaN for other b, so that every quotient fails
-// the range test; infinities give NaN too.
+// kQuotMax] when b lies in [2^-20, 2^40]: nothing overflows, and the remainder,
+// a multiple of 2^-133 there, is exact also where it is subnormal (which the
+// build's -ftz=false keeps).  rcp_for_quotients(b) is NaN for other b, so that
+// every quotient fails the range test; infinities give NaN too.
 constexpr float kQuotMin = 1.0e-20f, kQuotMax = 1.0e20f;
 
 __device__ __forceinline__ float rcp_for_quotients(float b) {
@@ -395,14 +396,16 @@ __device__ __forceinline__ void neighbour_row(const Env& e, const unsigned* __re
 // bits.  Per two-substep frame of settled pools, with one warp (10,000
 // particles) or one thread per particle testing and computing as it goes, and
 // now (the sort's launches included): 10,000 particles 169 -> 55 us, 40,000
-// 308 -> 97 us, 400,000 1830 -> 669 us.
+// 308 -> 97 us, 400,000 1830 -> 669 us.  Frames 20 to 70 of the fall of 400,000,
+// with up to twice the neighbours: 2170 -> 1070 us.
 // ---------------------------------------------------------------------------
 
-// Neighbours listed per particle (a settled pool has 25-60, its bottom up to
-// 100; a particle with more walks its rows again for the force: with 64, the
-// bottom's did, 400,000 particles 1165 instead of 758 us).  Entry k of sorted
-// particle s is nbr[k * stride + s], so that neighbouring particles' entries
-// share sectors.  No lists are kept for capacities above kListedMax, where
+// Neighbours listed per particle.  Of 400,000 particles at rest each has 36 on
+// average and at most 78; while they fall, 70 and at most 193, and in the densest
+// frame 3 % have more than 128.  A particle with more than are listed walks its
+// rows again for the force (with 64, those at the bottom of the settled pool did:
+// 1165 instead of 758 us).  Entry k of sorted particle s is nbr[k * stride + s],
+// so that neighbouring particles' entries share sectors.  No lists are kept for capacities above kListedMax, where
 // they would take over 4 GB, nor where there is no memory for them.
 constexpr int kNeighbours = 128;
 constexpr int kListedMax = 1 << 23;
