@@ -89,6 +89,7 @@ void fake_reset(size_t room) {
     g_elapsed = nullptr;
 }
 void fake_elapsed(float (*ms)(int)) { g_elapsed = ms; }
+void fake_room(size_t room) { g_room = room; }
 int fake_unordered() { return g_unordered; }
 size_t fake_used() { return g_used; }
 const char* fake_launched() { return g_launched.c_str(); }
@@ -125,7 +126,7 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void
 
 cudaError_t cudaMalloc(void** p, size_t bytes) {
     *p = nullptr;
-    if (bytes > g_room - g_used) return result(cudaErrorMemoryAllocation);
+    if (bytes > g_room || g_used > g_room - bytes) return result(cudaErrorMemoryAllocation);
     *p = std::calloc(bytes ? bytes : 1, 1);  // pages that nothing touches take no room
     if (!*p) return result(cudaErrorMemoryAllocation);
     g_used += bytes;

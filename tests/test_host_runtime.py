@@ -35,7 +35,7 @@ def fake(pkg, fake_lib, monkeypatch):
     monkeypatch.setattr(pkg._lib, "_lib", None)
     monkeypatch.setattr(pkg.build, "build", lambda *a, **k: fake_lib)
     lib = pkg._lib.load()
-    lib.fake_reset.argtypes = [ctypes.c_size_t]
+    lib.fake_reset.argtypes = lib.fake_room.argtypes = [ctypes.c_size_t]
     lib.fake_used.restype = ctypes.c_size_t
     lib.fake_launched.restype = ctypes.c_char_p
     lib.fake_reset(-1)
@@ -187,6 +187,13 @@ def _use_renderer(pkg):
     r.close()
 
 
+def _use_sph(pkg):
+    sim = pkg.SPHSimulator(None, None, 0.08, maxParticles=1000)
+    sim.upload(np.zeros((1000, 16), np.float32), [1.0, 2.0, 1.0])
+    sim.execute(SIDE_STREAM)
+    sim.close()
+
+
 @pytest.mark.parametrize("use", [
     _use_simulator, _use_batch, lambda pkg: _use_adjoint(pkg, "fp64"), lambda pkg: _use_adjoint(pkg, "fixed"),
     _use_renderer], ids=["simulator", "batch", "adjoint fp64", "adjoint fixed", "renderer"])
@@ -218,3 +225,23 @@ def test_autotune_chooses_by_the_longer_timing(fake, pkg):
     assert sim.tuning() == {"bin_pairing": 0, "task_threads": 256, "task_size": 512, "lane_table_min": 512}
     assert set(timed) == {1, 5}
     sim.close()
+
+
+@pytest.mark.parametrize("use", [
+    _use_simulator, _use_batch, lambda pkg: _use_adjoint(pkg, "fp64"), lambda pkg: _use_adjoint(pkg, "fixed"),
+    _use_renderer, _use_sph], ids=["simulator", "batch", "adjoint fp64", "adjoint fixed", "renderer", "sph"])
+def test_a_failed_call_leaves_no_error_behind(fake, pkg, use):
+    """Where memory runs out anywhere on the way, the call that fails says so,
+    and the next ones, with memory again, do not fail for it."""
+    failed = 0
+    room = 1 << 10
+    while room < 1 << 30:
+        fake.fake_room(room)
+        try:
+            use(pkg)
+        except pkg.MPMError:
+            failed += 1
+            fake.fake_room(1 << 40)
+            use(pkg)
+        room *= 2
+    assert failed > 3

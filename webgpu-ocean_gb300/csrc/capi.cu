@@ -81,8 +81,13 @@ int scene_lattice(float* out, int npa, double origin, double spacing, double jit
 }  // namespace
 
 namespace mpm {
-// Lets other translation units report a message through mpm_last_error().
-void set_last_error(const std::string& msg) { g_last_error = msg; }
+// Lets other translation units report a message through mpm_last_error().  The
+// runtime's last error goes with it: left there, the next call that looks for
+// its own launches' errors would fail for it.
+void set_last_error(const std::string& msg) {
+    g_last_error = msg;
+    cudaGetLastError();
+}
 
 // Reference 80-byte records in host memory <-> the library's four float4
 // streams, converted on the device: one copy of the records through a
